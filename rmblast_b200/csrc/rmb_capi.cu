@@ -20,6 +20,7 @@
 
 #include "../../include/rmb_gpu.h"
 #include "rmb_device.cuh"
+#include "rmb_dust.cuh"
 #include "rmb_glue.hpp"
 #include "rmb_kernels.hpp"
 
@@ -227,7 +228,10 @@ struct rmb_ctx {
     bool prelim_stream = false;  // thread-per-extension prelim kernel (else the warp kernel)
     rmb_tune tune = default_tune();  // launch knobs of the batched pipeline (rmb_tune_set / rmb_autotune)
     KaBlock ka;                  // E-value statistics (lambda <= 0: none)
-    DBuf dust_scratch, fails;    // per-thread DUST interval lists, their overflow flag
+    // DUST: the segments' units, converted bases, marks and per-query words; the bases that N draws;
+    // the sequential pass's interval lists and their overflow flag
+    DBuf dust_units, dust_conv, dust_mark, dust_words, dust_draws, dust_scratch, fails;
+    uint32_t n_dust_draws = 0;
     // the pipeline lanes: each a stream and the device buffers of one sub-batch at a time
     Work work[2];
     DevLib L{};
@@ -278,9 +282,67 @@ struct Taps {
     std::vector<uint32_t>* tracebacks = nullptr;  // strand, status, score, q0, q1, s0, s1, n_ops, ops hash
 };
 
+// DUST of a query set on the device (filter/dust.rs:462): the masked bases into qm (a copy of the
+// queries) and the interval bits, either of them null; in segments, then the sequential pass for the
+// queries that need it.  `compat` is the multi-chunk path's variant (engine.rs:697-707).
+void dust_queries(rmb_ctx& C, const rmb_queries& QH, uint8_t* qm, bool compat, uint32_t* bits,
+                  const uint64_t* bits_off, cudaStream_t st, rmb_counters& ctr) {
+    const uint32_t nq = QH.n;
+    const size_t bytes = QH.host.size();
+    uint64_t bases = 0;
+    for (uint32_t n : QH.len) bases += n;
+    const uint32_t seg = dust_segment_starts(bases, C.sms);
+    std::vector<uint32_t> unit_off(nq + 1, 0);
+    for (uint32_t i = 0; i < nq; ++i) unit_off[i + 1] = unit_off[i] + (QH.len[i] < 4 ? 0 : (QH.len[i] - 2 + seg - 1) / seg);
+    upload(C.dust_units, unit_off, st);
+    C.dust_conv.ensure(bytes);
+    C.dust_mark.ensure(bytes);
+    // per query: N count, flag; then the two control words
+    C.dust_words.ensure((2ull * nq + 2) * 4);
+    uint32_t* n_n = C.dust_words.as<uint32_t>();
+    uint32_t* flags = n_n + nq;
+    unsigned int* ctl = flags + nq;
+    unsigned int res[2] = {0, 0};
+    for (uint32_t want = 1u << 16;; want = res[1]) {
+        // the bases that N draws, in order (the same sequence for every query)
+        if (C.n_dust_draws < want) {
+            std::vector<uint8_t> draws(want);
+            DustRng rng;
+            rng.init();
+            for (uint8_t& d : draws) d = (uint8_t)(rng.get() & 3u);
+            upload(C.dust_draws, draws, st);
+            CK(cudaStreamSynchronize(st));
+            C.n_dust_draws = want;
+        }
+        CK(cudaMemsetAsync(C.dust_mark.p, 0, bytes, st));
+        CK(cudaMemsetAsync(flags, 0, (nq + 2ull) * 4, st));
+        if (qm) CK(cudaMemcpyAsync(qm, QH.d_q.p, bytes, cudaMemcpyDeviceToDevice, st));
+        CK(launch_dust_segments(QH.d_q.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq,
+                                C.dust_units.as<uint32_t>(), unit_off[nq], seg, C.dust_draws.as<uint8_t>(),
+                                C.n_dust_draws, C.dust_conv.as<uint8_t>(), n_n, C.dust_mark.as<uint8_t>(), flags, ctl,
+                                qm, compat, bits, bits_off, C.sms, st));
+        ctr.launches += 4;
+        CK(cudaMemcpyAsync(res, ctl, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (res[1] <= C.n_dust_draws) break;
+    }
+    if (!res[0]) return;
+    const uint32_t nt = dust_threads(nq, C.sms);
+    C.dust_scratch.ensure(dust_scratch_bytes(nt));
+    C.fails.ensure(16);
+    CK(cudaMemsetAsync(C.fails.p, 0, 4, st));
+    CK(launch_dust(QH.d_q.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq, qm, C.dust_scratch.p,
+                   nt, C.fails.as<unsigned int>(), compat, st, bits, bits_off, flags));
+    ctr.launches += 1;
+    unsigned int over = 0;
+    CK(cudaMemcpyAsync(&over, C.fails.p, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (over) throw Fail(RMB_ELIMIT, "DUST interval list outgrew its fixed capacity");
+}
+
 // DUST masking of a query set (engine.rs:606-616 -> filter/dust.rs:462), on the device: the
 // masked copy and its reverse complement feed the lookup tables and the exact word extension
-// only.  `compat` is the multi-chunk path's variant (engine.rs:697-707).
+// only.
 void mask_queries(rmb_ctx& C, rmb_queries& QH, bool compat, rmb_counters& ctr) {
     cudaStream_t st = C.st;
     const uint32_t nq = QH.n;
@@ -288,23 +350,14 @@ void mask_queries(rmb_ctx& C, rmb_queries& QH, bool compat, rmb_counters& ctr) {
     const size_t bytes = QH.host.size();
     QH.d_qm.ensure(bytes);
     QH.d_qmrc.ensure(bytes);
-    CK(cudaMemcpyAsync(QH.d_qm.p, QH.d_q.p, bytes, cudaMemcpyDeviceToDevice, st));
-    const uint32_t nt = dust_threads(nq, C.sms);
-    C.dust_scratch.ensure(dust_scratch_bytes(nt));
-    C.fails.ensure(16);
-    CK(cudaMemsetAsync(C.fails.p, 0, 4, st));
     EvTimer ev;
     ev.start(st);
-    CK(launch_dust(QH.d_q.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq, QH.d_qm.as<uint8_t>(),
-                   C.dust_scratch.p, nt, C.fails.as<unsigned int>(), compat, st));
+    dust_queries(C, QH, QH.d_qm.as<uint8_t>(), compat, nullptr, nullptr, st, ctr);
     CK(launch_revcomp(QH.d_qm.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq,
                       QH.d_qmrc.as<uint8_t>(), st));
     ev.stop(st);
-    ctr.launches += 2;
-    unsigned int over = 0;
-    CK(cudaMemcpyAsync(&over, C.fails.p, 4, cudaMemcpyDeviceToHost, st));
+    ctr.launches += 1;
     CK(cudaStreamSynchronize(st));
-    if (over) throw Fail(RMB_ELIMIT, "DUST interval list outgrew its fixed capacity");
     ctr.gpu_ms_dust += ev.ms();
     ctr.ms_lookup += ms_since(t0);
     QH.dusted = true;
@@ -2238,21 +2291,13 @@ int rmb_format_pairwise(rmb_ctx* C, const rmb_results* R, const uint8_t* const* 
             d_bits.ensure(std::max<uint64_t>(bits_off.back(), 1) * 4);
             upload(d_off, bits_off, C->st);
             CK(cudaMemsetAsync(d_bits.p, 0, std::max<uint64_t>(bits_off.back(), 1) * 4, C->st));
-            const uint32_t nt = dust_threads(R->n_queries, C->sms);
-            C->dust_scratch.ensure(dust_scratch_bytes(nt));
-            C->fails.ensure(16);
-            CK(cudaMemsetAsync(C->fails.p, 0, 4, C->st));
-            CK(launch_dust(QH->d_q.as<uint8_t>(), QH->d_off.as<uint64_t>(), QH->d_len.as<uint32_t>(), R->n_queries,
-                           nullptr, C->dust_scratch.p, nt, C->fails.as<unsigned int>(), false, C->st,
-                           d_bits.as<uint32_t>(), d_off.as<uint64_t>()));
+            rmb_counters ctr{};
+            dust_queries(*C, *QH, nullptr, false, d_bits.as<uint32_t>(), d_off.as<uint64_t>(), C->st, ctr);
             bits.resize(std::max<uint64_t>(bits_off.back(), 1));
-            unsigned int over = 0;
             CK(cudaMemcpyAsync(bits.data(), d_bits.p, bits.size() * 4, cudaMemcpyDeviceToHost, C->st));
-            CK(cudaMemcpyAsync(&over, C->fails.p, 4, cudaMemcpyDeviceToHost, C->st));
             CK(cudaStreamSynchronize(C->st));
             d_bits.release();
             d_off.release();
-            if (over) throw Fail(RMB_ELIMIT, "DUST interval list outgrew its fixed capacity");
         }
         std::string out;
         if (parts & 1) out += pairwise_header(db_name, C->ids.size(), C->total_letters);
@@ -2347,7 +2392,8 @@ void rmb_ctx_destroy(rmb_ctx* C) {
     if (!C) return;
     cudaSetDevice(C->p.device);
     DBuf* all[] = {&C->d_plus, &C->d_rc, &C->d_align, &C->d_align_rc, &C->d_packed, &C->d_plus_off, &C->d_packed_off,
-                   &C->d_len, &C->d_params, &C->lw, &C->dust_scratch, &C->fails, &C->sched_params};
+                   &C->d_len, &C->d_params, &C->lw, &C->dust_units, &C->dust_conv, &C->dust_mark,
+                   &C->dust_words, &C->dust_draws, &C->dust_scratch, &C->fails, &C->sched_params};
     for (DBuf* b : all) b->release();
     for (Work& w : C->work) w.release();
     if (C->batch) {

@@ -3,9 +3,9 @@
 //
 // One query is one sequential pass, as in the reference: the pass draws NCBI CRandom numbers for
 // N bases in order (dust.rs:24-57, 339-360) and restarts a window scan from the last window start
-// after each low-complexity run (dust.rs:400-460), so the masked positions depend on the whole
-// prefix.  The device runs one query per warp (one working lane); the queries of a batch run in
-// parallel.
+// after each homopolymer window (dust.rs:400-460), so the draws of later N depend on the whole
+// prefix.  The device takes the queries in segments (k_dust_segments in rmb_kernels.cu) and runs this
+// pass, one query per warp with one working lane, only for a query whose restart converts an N again.
 //
 // Storage differs from the reference's growable vectors, not the results:
 //  - the triplet list (at most window - 2 = 62 entries) is a 64-entry ring;

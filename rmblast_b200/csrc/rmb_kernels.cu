@@ -2726,18 +2726,300 @@ cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t
     return cudaGetLastError();
 }
 
-// DUST masking (filter/dust.rs:462-489).  A query's pass is one sequential chain of data-dependent
-// branches, so each query gets a warp of its own with one working lane: lanes of one warp on
-// different queries would diverge at nearly every step and run one after another.  Up to 32
-// such warps share an SM.  Each worker's perfect-interval list is in `scratch`; qm holds a copy
-// of q and gets the masked bases (code 14).
+// DUST masking (filter/dust.rs:462-489) in segments.  The reference's pass is sequential, but what
+// it masks is local: the interval it records for a start s is the longest [s, e] that scores above
+// the level and whose score density no interval inside it exceeds, over windows of 62 triplets, so
+// it depends on the bases of [s, s + 64) alone.  (The v suffix, `needs_processing` and the restart
+// after a window of one triplet only skip work: intervals inside v never reach the level, and a
+// restart scans the same starts again from the same bases.)  Two things are not local, and both
+// concern N, which draws a random base each time it is converted:
+//  - the draw of an N is the number of N before it (k_dust_convert's running count into the draws'
+//    fixed sequence);
+//  - the bases after a restart are converted again.  The restart at the end of the sequence is
+//    k_dust_segments<true>'s unit; one after a homopolymer window with an N in it shifts every later
+//    draw, so such a query is flagged and takes the sequential pass (k_dust).
+// Bound: the latency of a query's chain of steps.  k_dust's one working lane per query takes 0.65 us a
+// plain base and over 100 us one inside a simple repeat (searches of a 150 kb contig with 2 % simple
+// repeats: 808 ms, of 24 queries of 30 kb: 421 ms); a warp per 128 starts, its lanes on the 62 window
+// positions, makes a step's intervals by two warp scans (38 and 177 ms, the rest of the search).
+constexpr uint32_t DUST_TRIPLETS = DUST_WINDOW - 2;  // triplets in a full window
+constexpr uint32_t DUST_N_BASE = 0x80u;              // conv: the base was an N
+constexpr int DUST_CONVERT_BLOCK = 512, DUST_CONVERT_BASES = 16;
+
+// conv = the base codes DUST sees (dust_cvt), one block a query; n_n[qi] = the query's N count;
+// need = the draws the batch uses (draws past rnd_cap convert to 0: the caller grows rnd and runs
+// the batch again).
+__global__ void __launch_bounds__(DUST_CONVERT_BLOCK) k_dust_convert(
+    const uint8_t* __restrict__ q, const uint64_t* __restrict__ off, const uint32_t* __restrict__ len,
+    const uint8_t* __restrict__ rnd, uint32_t rnd_cap, uint8_t* __restrict__ conv, uint32_t* __restrict__ n_n,
+    unsigned int* __restrict__ need) {
+    __shared__ uint32_t warp_n[DUST_CONVERT_BLOCK / 32];
+    const uint64_t o = off[blockIdx.x] + 1;
+    const uint32_t n = len[blockIdx.x];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    constexpr uint32_t TILE = DUST_CONVERT_BLOCK * DUST_CONVERT_BASES;
+    uint32_t before = 0;  // N in the tiles so far
+    for (uint64_t t0 = 0; t0 < n; t0 += TILE) {
+        const uint64_t p0 = t0 + (uint64_t)threadIdx.x * DUST_CONVERT_BASES;
+        uint8_t b[DUST_CONVERT_BASES];
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < DUST_CONVERT_BASES; ++k) {
+            b[k] = p0 + k < n ? q[o + p0 + k] : 0;
+            c += b[k] == 14;
+        }
+        uint32_t incl = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        if (lane == 31) warp_n[wib] = incl;
+        __syncthreads();
+        uint32_t rank = before + incl - c, total = 0;
+#pragma unroll
+        for (int w = 0; w < DUST_CONVERT_BLOCK / 32; ++w) {
+            if (w < wib) rank += warp_n[w];
+            total += warp_n[w];
+        }
+        before += total;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < DUST_CONVERT_BASES; ++k) {
+            if (p0 + k >= n) break;
+            uint8_t v = b[k] < 4 ? b[k] : 0;
+            if (b[k] == 14) {
+                v = (uint8_t)(DUST_N_BASE | (rank < rnd_cap ? rnd[rank] : 0));
+                ++rank;
+            }
+            conv[o + p0 + k] = v;
+        }
+    }
+    if (threadIdx.x == 0) {
+        n_n[blockIdx.x] = before;
+        atomicMax(need, before + DUST_WINDOW);  // the last window's N are drawn once more
+    }
+}
+
+// One warp per unit: the intervals that start at the triplets [p0, p1) of a query, marked in mk.
+// A main unit (TAIL false) takes `seg` starts; a TAIL unit takes a query's last window again with
+// its N drawn anew, where the query has more than one window and an N in the last.  Lane l holds the
+// window positions whose offset from p0 is l or l + 32 (mod 64): their triplet, how often it comes
+// again up to the current step, and the densest interval that starts there with its end.  A step
+// adds one triplet; the score of the interval from a position is the sum of the counts from it on,
+// a scan in age order (age 0 the newest: lane (o - age) & 31).  Steps where no triplet of the window
+// comes five times have no interval above the level.
+template <bool TAIL>
+__global__ void __launch_bounds__(128) k_dust_segments(
+    const uint8_t* __restrict__ conv, const uint64_t* __restrict__ off, const uint32_t* __restrict__ len, uint32_t nq,
+    const uint32_t* __restrict__ unit_off, uint32_t n_units, uint32_t seg, const uint8_t* __restrict__ rnd,
+    uint32_t rnd_cap, const uint32_t* __restrict__ n_n, uint8_t* __restrict__ mk, uint32_t* __restrict__ flags,
+    unsigned int* __restrict__ n_flagged) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t u = warp; u < n_units; u += nwarps) {
+        uint32_t qi = u, p0 = 0, p1 = 0;
+        if (!TAIL) {
+            uint32_t lo = 0, hi = nq;  // the last query whose first unit is <= u
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) / 2;
+                if (unit_off[mid] <= u) lo = mid;
+                else hi = mid;
+            }
+            qi = lo;
+        }
+        const uint32_t n = len[qi];
+        if (n < 4) continue;
+        const uint32_t ntrip = n - 2;
+        const uint8_t* cv = conv + off[qi] + 1;
+        uint8_t* out = mk + off[qi] + 1;
+        int64_t marked = -1;  // bases up to here are marked, or belong to the main pass's last interval
+        uint32_t t0 = 0, t1 = 0;  // TAIL: the window's 64 bases, lane l's l and l + 32
+        if (TAIL) {
+            if (ntrip <= DUST_TRIPLETS) continue;
+            p0 = ntrip - DUST_TRIPLETS;
+            p1 = ntrip;
+            t0 = cv[p0 + lane];
+            t1 = cv[p0 + 32 + lane];
+            const unsigned m0 = __ballot_sync(FULL, t0 & DUST_N_BASE), m1 = __ballot_sync(FULL, t1 & DUST_N_BASE);
+            if (!(m0 | m1)) continue;  // the same bases: nothing new
+            const unsigned below = (1u << lane) - 1u;
+            const uint32_t r0 = n_n[qi] + __popc(m0 & below), r1 = n_n[qi] + __popc(m0) + __popc(m1 & below);
+            if (t0 & DUST_N_BASE) t0 = r0 < rnd_cap ? rnd[r0] : 0;
+            if (t1 & DUST_N_BASE) t1 = r1 < rnd_cap ? rnd[r1] : 0;
+            // an interval found now joins the last one of the main pass and only extends it
+            const unsigned k0 = __ballot_sync(FULL, out[p0 + lane]), k1 = __ballot_sync(FULL, out[p0 + 32 + lane]);
+            marked = k1 ? (int64_t)p0 + 63 - __clz((int)k1) : k0 ? (int64_t)p0 + 31 - __clz((int)k0) : (int64_t)p0 - 1;
+        } else {
+            p0 = (u - unit_off[qi]) * seg;
+            p1 = min(p0 + seg, ntrip);
+            marked = (int64_t)p0 - 1;
+        }
+        auto base = [&](uint32_t p) -> uint32_t { return p < n ? (uint32_t)cv[p] : 0u; };
+        auto mark = [&](uint32_t s, uint32_t e) {  // every lane together
+            for (int64_t x = max((int64_t)s, marked + 1) + lane; x <= (int64_t)e; x += 32) out[x] = 1;
+            marked = max(marked, (int64_t)e);
+        };
+        uint32_t trip[2] = {0xffu, 0xffu}, cnt[2] = {0, 0}, end[2] = {0, 0};
+        bool isn[2] = {false, false};
+        float den[2] = {-1.0f, -1.0f};
+        bool uniform = false;  // the window of the step before: full, of one triplet
+        uint32_t tb = 0, b_cur = 0, b_next = TAIL ? t0 : base(p0 + lane);
+        // one step past the last start's last interval, to see a homopolymer window end
+        const uint32_t last = min(p1 + DUST_TRIPLETS - 1, ntrip - 1);
+        for (uint32_t e = p0; e <= last; ++e) {
+            const uint32_t o = e - p0;
+            if ((o & 31) == 0) {
+                b_cur = b_next;
+                b_next = TAIL ? (o == 0 ? t1 : 0) : base(e + 32 + lane);
+                const uint32_t c1 = __shfl_sync(FULL, b_cur, (lane + 1) & 31), c2 = __shfl_sync(FULL, b_cur, (lane + 2) & 31);
+                const uint32_t n1 = __shfl_sync(FULL, b_next, (lane + 1) & 31), n2 = __shfl_sync(FULL, b_next, (lane + 2) & 31);
+                tb = ((b_cur & 3u) << 4) | (((lane < 31 ? c1 : n1) & 3u) << 2) | ((lane < 30 ? c2 : n2) & 3u) |
+                     (b_cur & DUST_N_BASE);
+            }
+            const uint32_t tn = __shfl_sync(FULL, tb, o & 31), t = tn & 63u;
+            if (o >= DUST_TRIPLETS) {  // the position that left the window
+                const uint32_t x = (o - DUST_TRIPLETS) & 63u;
+                const uint32_t xe = __shfl_sync(FULL, x >> 5 ? end[1] : end[0], x & 31);
+                if (xe && e - DUST_TRIPLETS < p1) mark(e - DUST_TRIPLETS, xe);
+                if (lane == (int)(x & 31)) {
+                    if (x >> 5) { trip[1] = 0xffu; cnt[1] = 0; den[1] = -1.0f; isn[1] = false; }
+                    else { trip[0] = 0xffu; cnt[0] = 0; den[0] = -1.0f; isn[0] = false; }
+                }
+            }
+            cnt[0] += trip[0] == t;
+            cnt[1] += trip[1] == t;
+            const bool nh = (o >> 5) & 1;  // the half that the new position's slot is in
+            if (lane == (int)(o & 31)) {
+                if (nh) { trip[1] = t; cnt[1] = 0; end[1] = 0; den[1] = -1.0f; isn[1] = tn >> 7; }
+                else { trip[0] = t; cnt[0] = 0; end[0] = 0; den[0] = -1.0f; isn[0] = tn >> 7; }
+            }
+            if (!__any_sync(FULL, max(cnt[0], cnt[1]) >= 4)) continue;
+            {
+                const uint32_t x = (o - (DUST_TRIPLETS - 1)) & 63u;
+                const bool now = o >= DUST_TRIPLETS - 1 &&
+                                 __shfl_sync(FULL, x >> 5 ? cnt[1] : cnt[0], x & 31) == DUST_TRIPLETS - 1;
+                if (uniform && !now && !TAIL) {
+                    // the reference restarts here: with an N in what it converts again, the draws shift
+                    const bool hit = __any_sync(FULL, isn[0] || isn[1]) ||
+                                     ((base(e + 1) | base(e + 2)) & DUST_N_BASE);
+                    if (hit && lane == 0 && atomicExch(flags + qi, 1u) == 0) atomicAdd(n_flagged, 1u);
+                }
+                uniform = now;
+            }
+            // by age: `young` is the slot of age ay, `old` that of age ay + 32
+            const uint32_t ay = (o - lane) & 31u;
+            const bool yh = lane <= (int)(o & 31) ? nh : !nh;
+            const uint32_t cy = yh ? cnt[1] : cnt[0], co = yh ? cnt[0] : cnt[1];
+            uint32_t x = cy | (co << 16);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_sync(FULL, x, (lane + d) & 31);
+                if (ay >= (uint32_t)d) x += v;
+            }
+            const uint32_t sy = x & 0xffffu, so = (x >> 16) + (__shfl_sync(FULL, x, (o + 1) & 31) & 0xffffu);
+            // score * 10 > level * (triplets - 1)
+            const bool can_y = cy > 0 && sy * 10 > DUST_LEVEL * ay, can_o = co > 0 && so * 10 > DUST_LEVEL * (ay + 32);
+            if (!__any_sync(FULL, can_y || can_o)) continue;
+            // densities as floats: two different score / length below 62 x 61 / 2 and 62 are further
+            // apart than a float's rounding, and equal ones round alike
+            const float ry = can_y ? __fdiv_rn((float)sy, (float)ay) : -1.0f;
+            const float ro = can_o ? __fdiv_rn((float)so, (float)(ay + 32)) : -1.0f;
+            const float py = yh ? den[1] : den[0], po = yh ? den[0] : den[1];
+            float qy = fmaxf(ry, py), qo = fmaxf(ro, po);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const float vy = __shfl_sync(FULL, qy, (lane + d) & 31), vo = __shfl_sync(FULL, qo, (lane + d) & 31);
+                if (ay >= (uint32_t)d) {
+                    qy = fmaxf(qy, vy);
+                    qo = fmaxf(qo, vo);
+                }
+            }
+            const float all_y = __shfl_sync(FULL, qy, (o + 1) & 31);
+            float ey = __shfl_sync(FULL, qy, (lane + 1) & 31), eo = __shfl_sync(FULL, qo, (lane + 1) & 31);
+            if (ay == 0) ey = eo = -1.0f;
+            eo = fmaxf(eo, all_y);
+            if (can_y && ry >= fmaxf(ey, py)) {
+                if (yh) { den[1] = ry; end[1] = e + 2; }
+                else { den[0] = ry; end[0] = e + 2; }
+            }
+            if (can_o && ro >= fmaxf(eo, po)) {
+                if (yh) { den[0] = ro; end[0] = e + 2; }
+                else { den[1] = ro; end[1] = e + 2; }
+            }
+        }
+        // the starts still in the window
+        const uint32_t o = last - p0;
+        for (uint32_t s = o >= DUST_TRIPLETS ? o - DUST_TRIPLETS + 1 : 0; s <= o && p0 + s < p1; ++s) {
+            const uint32_t xe = __shfl_sync(FULL, (s >> 5) & 1 ? end[1] : end[0], s & 31);
+            if (xe) mark(p0 + s, xe);
+        }
+    }
+}
+
+// The marked bases of the queries without a flag: masked in qm (with compat, also the base after
+// each interval) and as bits (zeros for a flagged query).
+__global__ void __launch_bounds__(256) k_dust_apply(const uint8_t* __restrict__ mk, const uint64_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ len, const uint32_t* __restrict__ flags,
+                                                    uint8_t* __restrict__ qm, bool compat, uint32_t* __restrict__ bits,
+                                                    const uint64_t* __restrict__ bits_off) {
+    const uint32_t qi = blockIdx.x;
+    const bool skip = flags[qi];  // the sequential pass's: nothing masked, no bits
+    const uint32_t n = len[qi];
+    const uint64_t o = off[qi] + 1;
+    const uint64_t t = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.y * blockDim.x;
+    if (qm && !skip)
+        for (uint64_t p = t; p < n; p += nt)
+            if (mk[o + p] || (compat && p > 0 && mk[o + p - 1])) qm[o + p] = 14;
+    if (bits)
+        for (uint64_t w = t; w * 32 < n; w += nt) {
+            uint32_t v = 0;
+            for (uint32_t b = 0; b < 32 && w * 32 + b < n && !skip; ++b)
+                if (mk[o + w * 32 + b]) v |= 1u << b;
+            bits[bits_off[qi] + w] = v;
+        }
+}
+
+uint32_t dust_segment_starts(uint64_t bases, int sms) {
+    // a unit scans 62 steps past its starts: short units while there are few (a 150 kb contig makes
+    // 1,172 units of 128), long ones once 128 would give every resident warp several
+    return bases / 128 > (uint64_t)sms * 64 * 4 ? 512u : 128u;
+}
+
+cudaError_t launch_dust_segments(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq,
+                                 const uint32_t* unit_off, uint32_t n_units, uint32_t seg, const uint8_t* rnd,
+                                 uint32_t rnd_cap, uint8_t* conv, uint32_t* n_n, uint8_t* mk, uint32_t* flags,
+                                 unsigned int* ctl, uint8_t* qm, bool compat, uint32_t* bits,
+                                 const uint64_t* bits_off, int sms, cudaStream_t st) {
+    if (!nq) return cudaSuccess;
+    k_dust_convert<<<nq, DUST_CONVERT_BLOCK, 0, st>>>(q, off, len, rnd, rnd_cap, conv, n_n, ctl + 1);
+    const int block = 128;
+    if (n_units)
+        k_dust_segments<false><<<grid_for((uint64_t)n_units * 32, block, 16, sms), block, 0, st>>>(
+            conv, off, len, nq, unit_off, n_units, seg, rnd, rnd_cap, n_n, mk, flags, ctl);
+    k_dust_segments<true><<<grid_for((uint64_t)nq * 32, block, 16, sms), block, 0, st>>>(
+        conv, off, len, nq, nullptr, nq, seg, rnd, rnd_cap, n_n, mk, flags, ctl);
+    const uint64_t per = (n_units * (uint64_t)seg / nq + 256 * 16 - 1) / (256 * 16);
+    k_dust_apply<<<dim3(nq, (unsigned)(per < 1 ? 1 : per > 1024 ? 1024 : per)), 256, 0, st>>>(mk, off, len, flags, qm,
+                                                                                             compat, bits, bits_off);
+    return cudaGetLastError();
+}
+
+// The sequential pass for the flagged queries: one chain of data-dependent branches a query, so
+// each query gets a warp of its own with one working lane (lanes of one warp on different queries
+// would diverge at nearly every step and run one after another).  Up to 32 such warps share an SM.
+// Each worker's perfect-interval list is in `scratch`; qm holds a copy of q and gets the masked
+// bases (code 14).
 __global__ void __launch_bounds__(32) k_dust(const uint8_t* __restrict__ q, const uint64_t* __restrict__ off,
                                              const uint32_t* __restrict__ len, uint32_t nq, uint8_t* __restrict__ qm,
                                              DustPerfect* __restrict__ scratch, uint32_t nworkers,
                                              unsigned int* __restrict__ overflow, bool compat,
-                                             uint32_t* __restrict__ bits, const uint64_t* __restrict__ bits_off) {
+                                             uint32_t* __restrict__ bits, const uint64_t* __restrict__ bits_off,
+                                             const uint32_t* __restrict__ flags) {
     if (threadIdx.x != 0 || blockIdx.x >= nworkers) return;
     for (uint32_t i = blockIdx.x; i < nq; i += nworkers) {
+        if (!flags[i]) continue;
         const uint64_t o = off[i] + 1;
         if (!dust_query(q + o, len[i], qm ? qm + o : nullptr, scratch + (uint64_t)blockIdx.x * DUST_PERFECT_CAP,
                         compat, bits ? bits + bits_off[i] : nullptr))
@@ -2753,10 +3035,10 @@ size_t dust_scratch_bytes(uint32_t nthreads) { return (size_t)nthreads * DUST_PE
 
 cudaError_t launch_dust(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint8_t* qm,
                         void* scratch, uint32_t nthreads, unsigned int* overflow, bool compat, cudaStream_t st,
-                        uint32_t* bits, const uint64_t* bits_off) {
+                        uint32_t* bits, const uint64_t* bits_off, const uint32_t* flags) {
     if (!nq || !nthreads) return cudaSuccess;
     k_dust<<<nthreads, 32, 0, st>>>(q, off, len, nq, qm, (DustPerfect*)scratch, nthreads, overflow, compat, bits,
-                                    bits_off);
+                                    bits_off, flags);
     return cudaGetLastError();
 }
 }  // namespace rmb

@@ -156,13 +156,25 @@ cudaError_t launch_lut_build(const DevQueries& Q, int32_t ws, uint32_t nq, const
 namespace rmb {
 cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint8_t* rc,
                            cudaStream_t st);
-// DUST masking of a query batch: qm must hold a copy of q; `scratch` holds
-// dust_scratch_bytes(nthreads); overflow counts queries whose interval list overflowed; compat
-// adds the multi-chunk path's extra masked base after each interval.  qm may be null; bits
-// (zeroed, per query at word offset bits_off[i]) gets one bit per position inside an interval.
+// DUST masking of a query batch in segments (k_dust_segments): unit_off[i] is query i's first unit of
+// `seg` starts (dust_segment_starts), rnd the first rnd_cap bases the N draw, conv, n_n, mk (zeroed),
+// flags (zeroed) and ctl (two zeroed words) scratch of the queries' layout or one word a query.  qm must
+// hold a copy of q and gets the masked bases; compat adds the multi-chunk path's extra masked base
+// after each interval; bits (per query at word offset bits_off[i]) one bit per position inside an
+// interval; either may be null.  After it ctl[0] counts the queries whose flag is set: nothing of
+// them is masked, launch_dust has to take them; ctl[1] the draws the batch needs: where that is over
+// rnd_cap, nothing holds and the batch runs again with more.
+uint32_t dust_segment_starts(uint64_t bases, int sms);
+cudaError_t launch_dust_segments(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq,
+                                 const uint32_t* unit_off, uint32_t n_units, uint32_t seg, const uint8_t* rnd,
+                                 uint32_t rnd_cap, uint8_t* conv, uint32_t* n_n, uint8_t* mk, uint32_t* flags,
+                                 unsigned int* ctl, uint8_t* qm, bool compat, uint32_t* bits,
+                                 const uint64_t* bits_off, int sms, cudaStream_t st);
+// The sequential pass over the flagged queries: `scratch` holds dust_scratch_bytes(nthreads);
+// overflow counts queries whose interval list overflowed.
 uint32_t dust_threads(uint32_t nq, int sms);
 size_t dust_scratch_bytes(uint32_t nthreads);
 cudaError_t launch_dust(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint8_t* qm,
                         void* scratch, uint32_t nthreads, unsigned int* overflow, bool compat, cudaStream_t st,
-                        uint32_t* bits = nullptr, const uint64_t* bits_off = nullptr);
+                        uint32_t* bits, const uint64_t* bits_off, const uint32_t* flags);
 }  // namespace rmb
