@@ -68,11 +68,13 @@ typedef struct rmb_ctx rmb_ctx;
  * only how work is laid out on the GPU).  rmb_ctx_create starts from the hand-swept defaults;
  * rmb_autotune times candidates on sample queries and keeps the fastest; rmb_tune_get/set read
  * and write them (a caller can persist and reuse a tuned set).
+ * The prelim_* knobs but prelim_window shape the thread-per-extension DP, which runs where the
+ * packed-row DP's number ranges do not hold (an X-drop over 128, scores near 127).
  *   prelim_group            cell steps a lane of the thread-per-extension DP runs between its
  *                           row-end blocks: 4, 8 or 16
  *   prelim_blocks_per_sm    resident blocks per SM of that DP's persistent grid, 1..6
- *   prelim_window           widest band, in cells, one thread keeps, 16..60: a wider extension is
- *                           handed to a warp (32 threads per alignment)
+ *   prelim_window           widest band, in cells, that DP or the packed-row DP keeps, 16..60: a
+ *                           wider extension is handed to a warp (32 threads per alignment)
  *   prelim_budget_div       DP cells one thread spends on a record before a warp takes it:
  *                           records / div, within 8,192 .. 2^20; 16..4096
  *   ungapped_blocks_per_sm  blocks per SM of the persistent ungapped-extension grid, 1..8

@@ -162,7 +162,7 @@ struct Work {
     DBuf pv, pv_off, cs, cs_off, cq, cq_off, pos_off, lut_keys, lut_vals, lut_keys2, lut_vals2, lut_counts;
     DBuf counts, offs, hits, hit_pair, ub, flags, dd_scratch, dd_cells, ung_idx, n_sel, po, wide, wide2, dres, geo,
         n_wide, band, sel, surv, cells, fails, temp, tb_in, tb_out, tb_ops, tb_scratch, stage, stage_start, stage_over,
-        tb_ooff, tb_ops2, ung_queue, dd_units, tb_half, tb_cells;
+        tb_ooff, tb_ops2, ung_queue, dd_units, tb_half, tb_cells, pack_list, pack_ctl;
     DBuf sched_pred, sched_order, sched_scratch, sched_feat, sched_cells;
     // the device chain as a CUDA graph (chain_graph): its executable, its timing events and the
     // pinned block its counts come back in
@@ -181,7 +181,7 @@ struct Work {
                        &lut_vals2, &lut_counts, &counts, &offs, &hits, &hit_pair, &ub, &flags, &dd_scratch, &dd_cells,
                        &ung_idx, &n_sel, &po, &wide, &wide2, &dres, &geo, &n_wide, &band, &sel, &surv, &cells, &fails,
                        &temp, &tb_in, &tb_out, &tb_ops, &tb_scratch, &stage, &stage_start, &stage_over, &tb_ooff,
-                       &tb_ops2, &ung_queue, &dd_units, &tb_half, &tb_cells, &sched_pred, &sched_order, &sched_scratch, &sched_feat, &sched_cells};
+                       &tb_ops2, &ung_queue, &dd_units, &tb_half, &tb_cells, &pack_list, &pack_ctl, &sched_pred, &sched_order, &sched_scratch, &sched_feat, &sched_cells};
         for (DBuf* b : all) b->release();
         if (st) cudaStreamDestroy(st);
         if (st2) cudaStreamDestroy(st2);
@@ -222,10 +222,13 @@ struct rmb_ctx {
     uint32_t max_slen = 0;
     bool loaded = false;
     // library, device
+    DBuf d_dp;  // the packed-row DP's copy of the library
     DBuf d_plus, d_rc, d_align, d_align_rc, d_packed, d_plus_off, d_packed_off, d_len, d_params;
     // the query set's lookup widths (read by every lane)
     DBuf lw;
     bool prelim_stream = false;  // thread-per-extension prelim kernel (else the warp kernel)
+    bool prelim_pack = false;    // within it, the packed-row kernels
+    bool prelim_dual = false;    // with k_prelim_dual before k_prelim_pack
     rmb_tune tune = default_tune();  // launch knobs of the batched pipeline (rmb_tune_set / rmb_autotune)
     KaBlock ka;                  // E-value statistics (lambda <= 0: none)
     // DUST: the segments' units, converted bases, marks and per-query words; the bases that N draws;
@@ -256,6 +259,9 @@ struct rmb_queries {
     DBuf d_q, d_qrc, d_off, d_len;
     DBuf d_qm, d_qmrc;   // DUST-masked queries and their reverse complements (made on first use)
     bool dusted = false;
+    DBuf d_dp;           // the packed-row DP's copies (made on first use)
+    uint64_t dp_stride = 0;
+    bool dp_made = false;
     void release() {
         d_q.release();
         d_qrc.release();
@@ -263,6 +269,7 @@ struct rmb_queries {
         d_len.release();
         d_qm.release();
         d_qmrc.release();
+        d_dp.release();
     }
 };
 
@@ -393,6 +400,29 @@ void finish_query(const rmb_ctx& C, std::vector<Hit>& v, uint32_t qlen) {
     sort_hit_list_order(v, C.ids);
 }
 
+// The packed-row DP's part of a launch shape: its sequence copies and, where k_prelim_dual runs
+// first, the list of up to n records between the two kernels.
+void pack_config(rmb_ctx& C, Work& W, const DevQueries& Q, uint64_t n, StreamLaunch& cfg) {
+    // the cell log covers the records that the thread-per-extension kernel completes
+    cfg.pack = C.prelim_pack && !C.sched_log;
+    cfg.dual = cfg.pack && C.prelim_dual;
+    if (cfg.pack) {
+        W.pack_ctl.ensure(16);
+        cfg.list_ctl = W.pack_ctl.as<unsigned int>();
+    }
+    if (cfg.dual) {
+        W.pack_list.ensure(std::max<uint64_t>(n, 1) * 4);
+        cfg.list = W.pack_list.as<uint32_t>();
+    }
+    cfg.cutoff = C.gp.gapped_cutoff;
+    cfg.gap_open = C.p.gap_open;
+    cfg.gap_extend = C.p.gap_extend;
+    cfg.q_dp = Q.dp;
+    cfg.s_dp = C.L.dp;
+    cfg.q_stride = Q.dp_stride;
+    cfg.s_stride = C.L.dp_stride;
+}
+
 // The batched pipeline's device chain of one pair range as one CUDA graph: the dedup with the
 // ungapped extension, the ungapped records' selection, the prelim DP geometry, the learned order,
 // the prelim DP with its warp fallback for the records it passes on, and the survivors' selection
@@ -453,6 +483,7 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     cfg.blocks_per_sm = tn.prelim_blocks_per_sm;
     cfg.window = tn.prelim_window;
     cfg.budget_div = tn.prelim_budget_div;
+    pack_config(C, W, Q, n1, cfg);
     auto rec = [&](int k) { CK(cudaEventRecordWithFlags(W.ev[k], st, cudaEventRecordExternal)); };
 
     cudaGraph_t g = nullptr;
@@ -479,7 +510,7 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
         rec(1);
         const unsigned int* nu_dev = W.n_sel.as<unsigned int>();
         CK(launch_prelim_prep(C.L, Q, C.d_params.as<DevParams>(), n1, W.ung_idx.as<uint32_t>(), W.hits.as<SeedHit>(),
-                              W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms, st, nu_dev));
+                              W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms, st, C.prelim_pack, nu_dev));
         const uint32_t* order = nullptr;
         rec(6);
         if (learned) {
@@ -665,6 +696,13 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
     cudaStream_t st = C.st;
     upload(C.lw, lw_all, st);
     if (P.dust && !QH.dusted && nq) mask_queries(C, QH, false, ctr);
+    if (C.prelim_pack && !QH.dp_made && nq) {
+        QH.dp_stride = dp_query_stride(QH.host.size(), nq);
+        QH.d_dp.ensure(dp_bytes(4, QH.dp_stride));
+        CK(launch_dp_query(QH.d_q.as<uint8_t>(), QH.d_qrc.as<uint8_t>(), QH.d_off.as<uint64_t>(),
+                           QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride, st));
+        QH.dp_made = true;
+    }
     const uint8_t* qmask = P.dust ? QH.d_qm.as<uint8_t>() : QH.d_q.as<uint8_t>();
     const uint8_t* qmask_rc = P.dust ? QH.d_qmrc.as<uint8_t>() : QH.d_qrc.as<uint8_t>();
     // Sub-batches of queries sharing one ungapped cutoff, bounded by lookup-table size; with two
@@ -727,7 +765,8 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
         DevQueries Q{QH.d_q.as<uint8_t>(),       QH.d_qrc.as<uint8_t>(),  qmask, qmask_rc,
                      QH.d_off.as<uint64_t>() + qb, QH.d_len.as<uint32_t>() + qb, W.pv.as<uint32_t>(),
                      W.pv_off.as<uint64_t>(),    W.cs.as<uint32_t>(),     W.cs_off.as<uint64_t>(),
-                     W.cq.as<uint32_t>(),        W.cq_off.as<uint64_t>(), C.lw.as<int32_t>() + qb, nb};
+                     W.cq.as<uint32_t>(),        W.cq_off.as<uint64_t>(), C.lw.as<int32_t>() + qb, nb,
+                     QH.d_dp.as<uint8_t>(),      QH.dp_stride,            qb};
         EvTimer ev;
         ev.start(st);
         {
@@ -1005,7 +1044,7 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
                 W.geo.ensure(std::max<uint64_t>(nu, 1) * prelim_geo_bytes());
                 CK(launch_prelim_prep(C.L, Q, C.d_params.as<DevParams>(), nu, W.ung_idx.as<uint32_t>(),
                                       W.hits.as<SeedHit>(), W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms,
-                                      st));
+                                      st, C.prelim_pack && !C.sched_log));
                 ctr.launches += nu ? 1 : 0;
                 const uint32_t* order = nullptr;
                 uint32_t* cells_out = nullptr;
@@ -1044,6 +1083,7 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
                 cfg.blocks_per_sm = tn.prelim_blocks_per_sm;
                 cfg.window = tn.prelim_window;
                 cfg.budget_div = tn.prelim_budget_div;
+                pack_config(C, W, Q, nu, cfg);
                 CK(launch_prelim_stream(C.d_params.as<DevParams>(), nu, W.geo.p, W.po.as<PrelimOut>(),
                                         W.wide.as<uint32_t>(), W.n_wide.as<unsigned int>(),
                                         W.cells.as<unsigned long long>(), C.sms, st, order, cells_out,
@@ -1556,6 +1596,8 @@ int rmb_ctx_create(const rmb_params* params, const int32_t scores[256], const do
         dp.gapped_cutoff = C->gp.gapped_cutoff;
         for (int i = 0; i < 256; ++i) dp.matrix[i] = scores[i];
         C->prelim_stream = p.kernels == 0 && prelim_stream_eligible(dp.matrix, p.gap_open, p.gap_extend, p.xdrop_gap);
+        C->prelim_pack = C->prelim_stream && prelim_pack_eligible(dp.matrix, p.gap_open, p.gap_extend, p.xdrop_gap);
+        C->prelim_dual = C->prelim_pack && prelim_dual_pays(dp.matrix, p.word_size, dp.gapped_cutoff);
         if (p.ka_lambda > 0.0) {
             if (!(p.ka_k > 0.0) || !(p.ka_h > 0.0) || !(p.ka_alpha > 0.0))
                 throw Fail(RMB_EINVAL, "statistics need K, H and alpha > 0 with lambda > 0");
@@ -1645,10 +1687,14 @@ int rmb_db_load(rmb_ctx* C, uint32_t n, const uint8_t* const* plus, const uint32
         upload(C->d_plus_off, C->plus_off, st);
         upload(C->d_packed_off, C->packed_off, st);
         upload(C->d_len, C->slen, st);
+        const uint64_t dp_stride = dp_subject_stride(hplus.size(), n);
+        C->d_dp.ensure(dp_bytes(2, dp_stride));
+        CK(launch_dp_subject(C->d_plus.as<uint8_t>(), C->d_plus_off.as<uint64_t>(), C->d_len.as<uint32_t>(), n,
+                             C->d_dp.as<uint8_t>(), dp_stride, st));
         CK(cudaStreamSynchronize(st));
         C->L = DevLib{C->d_plus.as<uint8_t>(),      C->d_rc.as<uint8_t>(),         C->d_align.as<uint8_t>(),
                       C->d_align_rc.as<uint8_t>(),  C->d_packed.as<uint8_t>(),     C->d_plus_off.as<uint64_t>(),
-                      C->d_packed_off.as<uint64_t>(), C->d_len.as<uint32_t>(), n};
+                      C->d_packed_off.as<uint64_t>(), C->d_len.as<uint32_t>(), n, C->d_dp.as<uint8_t>(), dp_stride};
         C->loaded = true;
         return RMB_OK;
     } catch (const Fail& e) {
@@ -1675,6 +1721,7 @@ static rmb_queries* make_queries(rmb_ctx* C, uint32_t nq, const uint8_t* const* 
     rmb_queries* H = into ? into : new rmb_queries();
     try {
         H->dusted = false;
+        H->dp_made = false;
         H->n = nq;
         H->device = C->p.device;
         H->len.assign(qlen, qlen + nq);
@@ -2391,7 +2438,7 @@ void rmb_text_free(void* p) { free(p); }
 void rmb_ctx_destroy(rmb_ctx* C) {
     if (!C) return;
     cudaSetDevice(C->p.device);
-    DBuf* all[] = {&C->d_plus, &C->d_rc, &C->d_align, &C->d_align_rc, &C->d_packed, &C->d_plus_off, &C->d_packed_off,
+    DBuf* all[] = {&C->d_dp, &C->d_plus, &C->d_rc, &C->d_align, &C->d_align_rc, &C->d_packed, &C->d_plus_off, &C->d_packed_off,
                    &C->d_len, &C->d_params, &C->lw, &C->dust_units, &C->dust_conv, &C->dust_mark,
                    &C->dust_words, &C->dust_draws, &C->dust_scratch, &C->fails, &C->sched_params};
     for (DBuf* b : all) b->release();

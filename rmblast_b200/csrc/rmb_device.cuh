@@ -20,6 +20,9 @@ struct DevLib {
     const uint64_t* packed_off;
     const uint32_t* len;
     uint32_t n;
+    // the packed-row DP's copy of plus (k_dp_subject), reversed at dp + dp_stride; or null
+    const uint8_t* dp = nullptr;
+    uint64_t dp_stride = 0;
 };
 
 // One batch of queries with their lookup tables.  Query i occupies off[i] .. off[i] + len[i] + 2
@@ -43,6 +46,11 @@ struct DevQueries {
     const uint64_t* cq_off;
     const int32_t* lw;
     uint32_t n;
+    // the packed-row DP's copies (k_dp_query) of q, q reversed, qrc and qrc reversed, dp_stride bytes
+    // apart; q0 is query 0's index in the query set, which its place in them depends on
+    const uint8_t* dp = nullptr;
+    uint64_t dp_stride = 0;
+    uint32_t q0 = 0;
 };
 
 struct DevParams {

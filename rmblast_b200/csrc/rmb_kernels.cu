@@ -24,6 +24,7 @@
 #include "rmb_device.cuh"
 #include "rmb_dust.cuh"
 #include "rmb_kernels.hpp"
+#include "rmb_prelim_dual.cuh"
 #include "rmb_prelim_stream.cuh"
 
 #include <cub/device/device_partition.cuh>
@@ -1443,7 +1444,7 @@ __global__ void __launch_bounds__(256) k_prelim_prep(DevLib L, DevQueries Q, con
                                                       const SeedHit* __restrict__ hits,
                                                       const uint32_t* __restrict__ hit_pair,
                                                       const UngBox* __restrict__ ub, PrelimGeo* __restrict__ geo,
-                                                      const unsigned int* __restrict__ n_dev) {
+                                                      bool pack, const unsigned int* __restrict__ n_dev) {
     if (n_dev) n = *n_dev;  // the count on the device (a graph-captured chain), n its capacity
     const int32_t goe = P->gap_open + P->gap_extend;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1456,7 +1457,54 @@ __global__ void __launch_bounds__(256) k_prelim_prep(DevLib L, DevQueries Q, con
         o.tbq = g.tbq; o.tbs = g.tbs;
         o.xdrop = (uint32_t)(g.xd > goe ? g.xd : goe);
         o.flags = (g.plus ? 1u : 0u) | ((uint32_t)al << 8) | ((uint32_t)ar << 16);
+        if (pack) {  // the packed-row DP reads its own copies of the sequences
+            const uint32_t pair = hit_pair[idx[t]], qi = pair / L.n, si = pair % L.n;
+            o.qseq = (uint64_t)(Q.dp + (g.plus ? 0 : 2 * Q.dp_stride) + Q.off[qi] + (uint64_t)PACK_PAD * (Q.q0 + qi + 1));
+            o.sseq = (uint64_t)(L.dp + L.plus_off[si] + (uint64_t)PACK_SPAD * (si + 1));
+        }
         geo[t] = o;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_dp_subject(const uint8_t* __restrict__ plus, const uint64_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ len, uint8_t* __restrict__ out,
+                                                    uint64_t stride) {
+    const uint64_t o = off[blockIdx.x];
+    const uint32_t n = len[blockIdx.x];
+    uint8_t* d = out + o + (uint64_t)PACK_SPAD * (blockIdx.x + 1);
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint8_t v = (uint8_t)((plus[o + 1 + i] & 15u) * 8u);
+        d[i] = v;
+        d[stride + n - 1 - i] = v;
+    }
+}
+
+// The codes of a byte copy, eight to a word: bits sh .. sh + 3 of each byte.
+__global__ void __launch_bounds__(256) k_dp_nibbles(const uint2* __restrict__ in, uint64_t n_words, int sh,
+                                                    uint32_t* __restrict__ out) {
+    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words; w += (uint64_t)gridDim.x * blockDim.x) {
+        uint2 v = in[w];
+        v.x = (v.x >> sh) & 0x0f0f0f0fu;
+        v.y = (v.y >> sh) & 0x0f0f0f0fu;
+        v.x |= v.x >> 4;
+        v.y |= v.y >> 4;
+        out[w] = prmt(prmt(v.x, 0, 0x4420), prmt(v.y, 0, 0x4420), 0x5410);
+    }
+}
+
+// Blocks (query, part of it); the bytes between the queries are filled by the caller.
+__global__ void __launch_bounds__(256) k_dp_query(const uint8_t* __restrict__ q, const uint8_t* __restrict__ qrc,
+                                                  const uint64_t* __restrict__ off, const uint32_t* __restrict__ len,
+                                                  uint8_t* __restrict__ out, uint64_t stride) {
+    const uint64_t o = off[blockIdx.x];
+    const uint32_t n = len[blockIdx.x];
+    uint8_t* d = out + o + (uint64_t)PACK_PAD * (blockIdx.x + 1);
+    for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.y * blockDim.x) {
+        const uint8_t f = (uint8_t)pack_sel(q[o + 1 + i] & 15u), r = (uint8_t)pack_sel(qrc[o + 1 + i] & 15u);
+        d[i] = f;
+        d[stride + n - 1 - i] = f;
+        d[2 * stride + i] = r;
+        d[3 * stride + n - 1 - i] = r;
     }
 }
 
@@ -2314,15 +2362,135 @@ bool prelim_stream_eligible(const int32_t* matrix256, int32_t gap_open, int32_t 
     return true;
 }
 
+// The widest initial row has to fit the window right of the pivot's diagonal, scores with both gap
+// decays a signed byte, and a blocked column's score of -128 has to end every path.
+bool prelim_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop_gap) {
+    const int32_t goe = gap_open + gap_extend, xmax = std::max(xdrop_gap, goe);
+    if (gap_extend < 1 || gap_open < 0 || xmax > PACK_XMAX) return false;
+    if ((xmax - goe) / gap_extend + 1 > 16) return false;
+    for (int a = 0; a < 16; ++a)
+        for (int b : {0, 1, 2, 3, 14})
+            if (matrix256[a * 16 + b] + 2 * gap_extend > 127) return false;
+    return true;
+}
+
+uint64_t dp_subject_stride(uint64_t bytes, uint32_t n) { return (bytes + (uint64_t)PACK_SPAD * (n + 1) + 15) & ~15ull; }
+uint64_t dp_query_stride(uint64_t bytes, uint32_t nq) { return (bytes + (uint64_t)PACK_PAD * (nq + 1) + 15) & ~15ull; }
+
+// the nibble words after the byte copies (64 bytes of slack: a code is read with the seven after it)
+const uint32_t* dp_nibbles(const uint8_t* dp, int copies, uint64_t stride) {
+    return reinterpret_cast<const uint32_t*>(dp + copies * stride);
+}
+uint64_t dp_bytes(int copies, uint64_t stride) { return copies * stride + copies * stride / 2 + 64; }
+
+// A record that reaches the cutoff runs twice, so k_prelim_dual pays where few do: with a cutoff of
+// 200 and word hits of 110 one in 2,000 does, with the default cutoff of 1 99 in 100 do.
+bool prelim_dual_pays(const int32_t* matrix256, int32_t word_size, int32_t gapped_cutoff) {
+    int32_t best = 0;
+    for (int a = 0; a < 4; ++a)
+        for (int b = 0; b < 4; ++b) best = std::max(best, matrix256[a * 16 + b]);
+    return gapped_cutoff > word_size * best;
+}
+
+// 8 lanes an extension: a row's chain is 4 registers and 3 shuffle steps (4 lanes of 8 registers
+// measured 4.4 ms on the longest alignments of a 100 kb genome, 8 of 4 with the sides apart 3.3)
+constexpr int PACK_G = 8, PACK_R = 4;
+
+static cudaError_t pack_launch(const DevParams* P, uint64_t n, const PrelimGeo* geo, PrelimOut* out, uint32_t* wide,
+                               unsigned int* n_wide, unsigned long long* cells, int sms, cudaStream_t st,
+                               const uint32_t* order, uint32_t* cells_out, bool plain, const StreamLaunch& cfg,
+                               const StreamDevCounts& dc, uint32_t window) {
+    // per-SM residency of the persistent grids (the same for every device: one architecture)
+    static const int dual_sm = [] {
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_prelim_dual<true>, DUAL_BLOCK, 0);
+        return std::max(b, 1);
+    }();
+    static const int pack_sm = [] {
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_prelim_pack<PACK_G, PACK_R>, PACK_BLOCK, 0);
+        return std::max(b, 1);
+    }();
+    const uint32_t* list = cfg.dual ? cfg.list : nullptr;
+    cudaError_t e = cudaMemsetAsync(cfg.list_ctl, 0, 8, st);
+    if (e != cudaSuccess) return e;
+    if (cfg.dual) {
+        DualConst K;
+        K.q_stride = cfg.q_stride;
+        K.s_stride = cfg.s_stride;
+        K.q_dp = cfg.q_dp;
+        K.s_dp = cfg.s_dp;
+        K.q_nib = dp_nibbles(cfg.q_dp, 4, cfg.q_stride);
+        K.s_nib = dp_nibbles(cfg.s_dp, 2, cfg.s_stride);
+        K.neg_go = pack2(-cfg.gap_open, -cfg.gap_open);
+        for (int c = 0; c < DUAL_W; ++c) {
+            K.neg_ge[c] = pack2(-cfg.gap_extend * c, -cfg.gap_extend * c);
+            K.pos_ge[c] = pack2(cfg.gap_extend * c, cfg.gap_extend * c);
+        }
+        K.one = 1;
+        K.minus_one = 0xffffffffu;
+        const uint64_t want = (n + 2 * DUAL_BLOCK - 1) / (2 * DUAL_BLOCK), cap = (uint64_t)sms * dual_sm;
+        if (plain)
+            k_prelim_dual<false><<<(unsigned)want, DUAL_BLOCK, 0, st>>>(P, K, n, geo, out, cfg.list, cfg.list_ctl, n_wide + 1,
+                                                                        cells, order, cells_out, window, dc);
+        else
+            k_prelim_dual<true><<<(unsigned)std::min(want, cap), DUAL_BLOCK, 0, st>>>(
+                P, K, n, geo, out, cfg.list, cfg.list_ctl, n_wide + 1, cells, order, cells_out, window, dc);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    PackConst<PACK_R> K;
+    K.q_stride = cfg.q_stride;
+    K.s_stride = cfg.s_stride;
+    K.neg_go = pack2(-cfg.gap_open, -cfg.gap_open);
+    for (int r = 0; r < PACK_R; ++r) {
+        K.neg_ge[r] = pack2(-cfg.gap_extend * r, -cfg.gap_extend * r);
+        K.live[r] = 0x80008000u - (uint32_t)(cfg.gap_extend * r) * 0x00010001u;
+    }
+    constexpr int GROUPS = PACK_BLOCK / PACK_G;
+    const uint64_t want = (2 * n + GROUPS - 1) / GROUPS, cap = (uint64_t)sms * pack_sm;
+    k_prelim_pack<PACK_G, PACK_R><<<(unsigned)std::min(want, cap), PACK_BLOCK, 0, st>>>(
+        P, K, n, geo, out, cfg.list_ctl + 1, STREAM_MAX_CELLS, window, dc.n, list, cfg.list_ctl);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_prelim_pack_join<<<grid_for(list ? std::min<uint64_t>(n, 1u << 18) : n, 256, 8, sms), 256, 0, st>>>(
+        n, geo, out, cfg.cutoff, wide, n_wide, cells, cells_out, dc.n, list, cfg.list_ctl);
+    return cudaGetLastError();
+}
+
 size_t prelim_geo_bytes() { return sizeof(PrelimGeo); }
 
 cudaError_t launch_prelim_prep(const DevLib& L, const DevQueries& Q, const DevParams* P, uint64_t n,
                                const uint32_t* idx, const SeedHit* hits, const uint32_t* hit_pair, const UngBox* ub,
-                               void* geo, int sms, cudaStream_t st, const unsigned int* n_dev) {
+                               void* geo, int sms, cudaStream_t st, bool pack, const unsigned int* n_dev) {
     if (!n) return cudaSuccess;
-    k_prelim_prep<<<grid_for(n, 256, 8, sms), 256, 0, st>>>(L, Q, P, n, idx, hits, hit_pair, ub, (PrelimGeo*)geo,
+    k_prelim_prep<<<grid_for(n, 256, 8, sms), 256, 0, st>>>(L, Q, P, n, idx, hits, hit_pair, ub, (PrelimGeo*)geo, pack,
                                                             n_dev);
     return cudaGetLastError();
+}
+
+static cudaError_t dp_pack(uint8_t* dp, int copies, uint64_t stride, int sh, cudaStream_t st) {
+    const uint64_t n = copies * stride / 8;
+    k_dp_nibbles<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 8192), 256, 0, st>>>(
+        (const uint2*)dp, n, sh, const_cast<uint32_t*>(dp_nibbles(dp, copies, stride)));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const uint32_t* len, uint32_t n, uint8_t* out,
+                              uint64_t stride, cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(out, 15 * 8, 2 * stride, st);
+    if (e != cudaSuccess) return e;
+    k_dp_subject<<<n, 256, 0, st>>>(plus, off, len, out, stride);
+    return dp_pack(out, 2, stride, 3, st);
+}
+
+cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t* off, const uint32_t* len, uint32_t nq,
+                            uint8_t* out, uint64_t stride, cudaStream_t st) {
+    if (!nq) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(out, PACK_BLOCKED, 4 * stride, st);
+    if (e != cudaSuccess) return e;
+    const uint64_t parts = stride / nq / 4096 + 1;
+    k_dp_query<<<dim3(nq, (unsigned)std::min<uint64_t>(parts, 1024)), 256, 0, st>>>(q, qrc, off, len, out, stride);
+    return dp_pack(out, 4, stride, 0, st);
 }
 
 cudaError_t launch_prelim_stream(const DevParams* P, uint64_t n, const void* geo, PrelimOut* out, uint32_t* wide,
@@ -2344,6 +2512,8 @@ cudaError_t launch_prelim_stream(const DevParams* P, uint64_t n, const void* geo
                                                   : budget > STREAM_MAX_CELLS ? STREAM_MAX_CELLS : budget);
     const uint32_t window = cfg.window < 1 ? 1 : cfg.window > STREAM_WINDOW ? STREAM_WINDOW : (uint32_t)cfg.window;
     const PrelimGeo* g = (const PrelimGeo*)geo;
+    if (cfg.pack)
+        return pack_launch(P, n, g, out, wide, n_wide, cells, sms, st, order, cells_out, plain, cfg, dc, window);
 #define RMB_STREAM_LAUNCH(U)                                                                                      \
     do {                                                                                                         \
         if (plain) /* one record per thread, the whole grid at once */                                           \

@@ -46,12 +46,13 @@ cudaError_t launch_prelim(const DevLib& L, const DevQueries& Q, const DevParams*
 // Whether the thread-per-extension kernel's int16 band entries and int8 score rows hold the
 // parameters exactly (scores <= 127; X-drop and gap_open + gap_extend <= 8000).
 // launch_prelim_stream uses n_wide[0] (overflow count) and n_wide[1] (record queue), both zeroed.
+bool prelim_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop_gap);
 bool prelim_stream_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop_gap);
 // geo: n x prelim_geo_bytes() of scratch for the per-record geometry.
 size_t prelim_geo_bytes();
 cudaError_t launch_prelim_prep(const DevLib& L, const DevQueries& Q, const DevParams* P, uint64_t n,
                                const uint32_t* idx, const SeedHit* hits, const uint32_t* hit_pair, const UngBox* ub,
-                               void* geo, int sms, cudaStream_t st, const unsigned int* n_dev = nullptr);
+                               void* geo, int sms, cudaStream_t st, bool pack, const unsigned int* n_dev = nullptr);
 // Launch shape of the thread-per-extension DP (from rmb_tune): group of cell steps between
 // row-end blocks (4, 8, 16), resident blocks per SM, widest band a thread keeps, cell budget divisor.
 // Counts a graph-captured chain keeps on the device: the DP's record count (its cell budget then
@@ -72,7 +73,27 @@ struct StreamDevCounts {
 };
 struct StreamLaunch {
     int group = 8, blocks_per_sm = 6, window = 60, budget_div = 128;
+    // the packed-row kernels (prelim_pack_eligible parameters): k_prelim_pack, after k_prelim_dual where
+    // `dual` is set (prelim_dual_pays), with a list of n entries and two words between them
+    bool pack = false, dual = false;
+    uint32_t* list = nullptr;
+    unsigned int* list_ctl = nullptr;
+    int gap_open = 0, gap_extend = 0, cutoff = 0;
+    const uint8_t *q_dp = nullptr, *s_dp = nullptr;  // the DP copies (DevQueries, DevLib)
+    uint64_t q_stride = 0, s_stride = 0;
 };
+// k_prelim_dual settles the records under the gapped cutoff: it pays where a word hit alone does not
+// reach it.
+bool prelim_dual_pays(const int32_t* matrix256, int32_t word_size, int32_t gapped_cutoff);
+// The packed-row DP's copies of the sequences, dp_bytes(copies, stride) bytes: the library's two
+// (bytes from plus, and reversed) and a query set's four (q and qrc, each also reversed).
+uint64_t dp_bytes(int copies, uint64_t stride);
+uint64_t dp_subject_stride(uint64_t bytes, uint32_t n);
+cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const uint32_t* len, uint32_t n, uint8_t* out,
+                              uint64_t stride, cudaStream_t st);
+uint64_t dp_query_stride(uint64_t bytes, uint32_t nq);
+cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t* off, const uint32_t* len, uint32_t nq,
+                            uint8_t* out, uint64_t stride, cudaStream_t st);
 cudaError_t launch_prelim_stream(const DevParams* P, uint64_t n, const void* geo, PrelimOut* out, uint32_t* wide,
                                  unsigned int* n_wide, unsigned long long* cells, int sms, cudaStream_t st,
                                  const uint32_t* order, uint32_t* cells_out, bool plain, const StreamLaunch& cfg,
