@@ -372,6 +372,7 @@ void mask_queries(rmb_ctx& C, rmb_queries& QH, bool compat, rmb_counters& ctr) {
 
 // One (query, subject) pair's Phase 2a output, in the reference's order (purge order).
 constexpr uint64_t MAX_RANGE_HITS = 1ull << 29;
+constexpr uint32_t BUCKET_DENSE_HITS = 8192;  // word hits a pair from which a dense range takes the bucket replay
 constexpr uint64_t SCHED_NF_HOST = 12;  // features per record of the learned schedule (rmb_sched.cuh)
 
 struct PairPrelims {
@@ -449,15 +450,24 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     W.flags.ensure(nh + 1);
     W.dd_cells.ensure(n1 * diag_cell_bytes());
     W.ung_queue.ensure(16);
-    if (!fused) W.dd_scratch.ensure(dedup_threads(C.sms) * 1024 * 4);
-    else W.dd_units.ensure(dedup_units_bytes(npairs, nh, C.sms));
+    const rmb_tune& tn = C.tune;
+    // The bucket replay, of all hits extended first or, in dense ranges, of the leaders.  k_dedup_extend
+    // keeps the dense ranges whose pairs hold few thousand hits: it extends no dropped hit, and a warp a
+    // pair is enough lanes there (50 queries of 5 kb against 300 of their own, 4,700 hits a pair: 21 ms
+    // to 27); over 8,192 hits a pair its rounds wait on one pair's buckets (100 kb against 50 consensi,
+    // 31,000 hits a pair: 10.6 ms to 0.9; two of 60 kb against 2,000, 20,000: 51 to 34).
+    const bool bucket_fits = bucket_dedup_fits(npairs, nh);
+    const bool leaders = fused && bucket_fits && nh >= (uint64_t)BUCKET_DENSE_HITS * npairs;
+    const bool buckets = bucket_fits && (leaders || !fused);
+    if (!fused && !buckets) W.dd_scratch.ensure(dedup_threads(C.sms) * 1024 * 4);
+    if (fused && !leaders) W.dd_units.ensure(dedup_units_bytes(npairs, nh, C.sms));
     W.ung_idx.ensure(n1 * 4);
     W.n_sel.ensure(16);   // [0] ungapped records, [1] survivors
     W.n_wide.ensure(16);  // [0] records the thread kernel passed on, [1] its queue, [2] those the warp kernel did
     W.cells.ensure(16);   // [0] DP cells, [1] the thread kernel's alone
     W.fails.ensure(16);
     W.po.ensure(n1 * sizeof(PrelimOut));
-    W.geo.ensure(n1 * prelim_geo_bytes());
+    W.geo.ensure(std::max(n1 * prelim_geo_bytes(), bucket_dedup_bytes(n1)));  // the dedup's sort, then the geometry
     W.wide.ensure(n1 * 4);
     W.wide2.ensure(wcap * 4);
     W.dres.ensure(wcap * 2 * sizeof(int4));
@@ -473,11 +483,14 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
                         st));
     CK(launch_select_prelim(W.po.as<PrelimOut>(), n1, W.sel.as<uint32_t>(), W.n_sel.as<uint32_t>() + 1, nullptr, t_pre,
                             st, W.n_sel.as<unsigned int>()));
-    W.temp.ensure(std::max(t_eq, std::max(t_pre, t_front)));
+    size_t t_bucket = 0;
+    if (buckets)
+        CK(launch_bucket_dedup(C.L, Q, nullptr, P.word_size, ucut, pair0, npairs, nh, nullptr, nullptr, nullptr, nullptr,
+                               nullptr, nullptr, 0, leaders, nullptr, nullptr, t_bucket, C.sms, st));
+    W.temp.ensure(std::max(std::max(t_eq, t_bucket), std::max(t_pre, t_front)));
     W.hcount.resize(64);
     for (cudaEvent_t& e : W.ev)
         if (!e) CK(cudaEventCreate(&e));
-    const rmb_tune& tn = C.tune;
     StreamLaunch cfg;
     cfg.group = tn.prelim_group;
     cfg.blocks_per_sm = tn.prelim_blocks_per_sm;
@@ -493,7 +506,12 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
         CK(cudaMemsetAsync(W.cells.p, 0, 16, st));
         CK(cudaMemsetAsync(W.fails.p, 0, 16, st));
         rec(0);
-        if (fused) {
+        if (leaders) {
+            CK(launch_bucket_dedup(C.L, Q, C.d_params.as<DevParams>(), P.word_size, ucut, pair0, npairs, nh,
+                                   W.hits.as<SeedHit>(), W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(),
+                                   W.flags.as<uint8_t>(), W.dd_cells.p, W.ung_queue.as<unsigned long long>(),
+                                   tn.ungapped_blocks_per_sm, true, W.geo.p, W.temp.p, t_bucket, C.sms, st));
+        } else if (fused) {
             CK(launch_dedup_extend(C.L, Q, C.d_params.as<DevParams>(), ucut, pair0, npairs, nh, W.offs.as<uint64_t>(),
                                    W.hits.as<SeedHit>(), W.ub.as<UngBox>(), W.flags.as<uint8_t>(), W.dd_cells.p,
                                    W.ung_queue.as<unsigned long long>(), W.dd_units.p, C.sms, st));
@@ -501,9 +519,14 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
             CK(launch_ungapped(C.L, Q, C.d_params.as<DevParams>(), ucut, nh, W.hits.as<SeedHit>(),
                                W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), C.sms, st,
                                W.ung_queue.as<unsigned long long>(), tn.ungapped_blocks_per_sm));
-            CK(launch_dedup(C.L, Q, P.word_size, ucut, pair0, npairs, W.offs.as<uint64_t>(), W.hits.as<SeedHit>(),
-                            W.ub.as<UngBox>(), W.flags.as<uint8_t>(), W.dd_scratch.as<uint32_t>(), W.dd_cells.p,
-                            C.sms, st));
+            if (buckets)
+                CK(launch_bucket_dedup(C.L, Q, nullptr, P.word_size, ucut, pair0, npairs, nh, W.hits.as<SeedHit>(),
+                                       W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.flags.as<uint8_t>(), W.dd_cells.p,
+                                       nullptr, 0, false, W.geo.p, W.temp.p, t_bucket, C.sms, st));
+            else
+                CK(launch_dedup(C.L, Q, P.word_size, ucut, pair0, npairs, W.offs.as<uint64_t>(), W.hits.as<SeedHit>(),
+                                W.ub.as<UngBox>(), W.flags.as<uint8_t>(), W.dd_scratch.as<uint32_t>(), W.dd_cells.p,
+                                C.sms, st));
         }
         CK(launch_select_eq(W.flags.as<uint8_t>(), nh, 3, W.ung_idx.as<uint32_t>(), W.n_sel.as<uint32_t>(), W.temp.p,
                             t_eq, st));
@@ -932,11 +955,25 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
                 ctr.ms_ungapped += ms_since(t0);
                 t0 = std::chrono::steady_clock::now();
                 W.flags.ensure(nh + 1);
-                W.dd_scratch.ensure(dedup_threads(C.sms) * 1024 * 4);
                 W.dd_cells.ensure(std::max<uint64_t>(nh, 1) * diag_cell_bytes());
-                ev.start(st);
-                CK(launch_dedup(C.L, Q, P.word_size, ucut[qb], pair0, npairs, W.offs.as<uint64_t>(), W.hits.as<SeedHit>(),
-                                W.ub.as<UngBox>(), W.flags.as<uint8_t>(), W.dd_scratch.as<uint32_t>(), W.dd_cells.p, C.sms, st));
+                if (P.pipeline != 1 && bucket_dedup_fits(npairs, nh)) {
+                    tb = 0;
+                    W.geo.ensure(bucket_dedup_bytes(nh));
+                    CK(launch_bucket_dedup(C.L, Q, nullptr, P.word_size, ucut[qb], pair0, npairs, nh, nullptr, nullptr,
+                                           nullptr, nullptr, nullptr, nullptr, 0, false, nullptr, nullptr, tb, C.sms, st));
+                    W.temp.ensure(tb);
+                    ev.start(st);
+                    CK(launch_bucket_dedup(C.L, Q, nullptr, P.word_size, ucut[qb], pair0, npairs, nh,
+                                           W.hits.as<SeedHit>(), W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(),
+                                           W.flags.as<uint8_t>(), W.dd_cells.p, nullptr, 0, false, W.geo.p, W.temp.p, tb,
+                                           C.sms, st));
+                } else {
+                    W.dd_scratch.ensure(dedup_threads(C.sms) * 1024 * 4);
+                    ev.start(st);
+                    CK(launch_dedup(C.L, Q, P.word_size, ucut[qb], pair0, npairs, W.offs.as<uint64_t>(),
+                                    W.hits.as<SeedHit>(), W.ub.as<UngBox>(), W.flags.as<uint8_t>(),
+                                    W.dd_scratch.as<uint32_t>(), W.dd_cells.p, C.sms, st));
+                }
                 ev.stop(st);
                 ctr.launches += 1;
             }

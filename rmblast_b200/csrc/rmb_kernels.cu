@@ -28,6 +28,8 @@
 #include "rmb_prelim_stream.cuh"
 
 #include <cub/device/device_partition.cuh>
+#include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_select.cuh>
 #include <thrust/iterator/counting_iterator.h>
 #include "rmb_sched.cuh"
 #include "rmb_ungapped.cuh"
@@ -319,7 +321,10 @@ template <bool QUEUE>
 __global__ void __launch_bounds__(256) k_ungapped(DevLib L, DevQueries Q, const DevParams* __restrict__ P,
                                                    int32_t ucut, uint64_t n, const SeedHit* __restrict__ hits,
                                                    const uint32_t* __restrict__ hit_pair, UngBox* __restrict__ out,
-                                                   unsigned long long* __restrict__ queue) {
+                                                   unsigned long long* __restrict__ queue,
+                                                   const uint32_t* __restrict__ list,
+                                                   const unsigned int* __restrict__ n_list) {
+    if (list) n = *n_list;  // the listed hits only
     __shared__ int32_t mat[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) mat[i] = P->matrix[i];
     __syncthreads();
@@ -351,6 +356,7 @@ __global__ void __launch_bounds__(256) k_ungapped(DevLib L, DevQueries Q, const 
                 if (i >= n) {
                     phase = 3;
                 } else {
+                    if (list) i = list[i] & 0x7fffffffu;
                     h = hits[i];
                     const uint32_t pair = hit_pair[i];
                     const uint32_t qi = pair / L.n, si = pair % L.n;
@@ -462,6 +468,184 @@ __global__ void __launch_bounds__(128) k_dedup(DevLib L, DevQueries Q, int32_t w
         const uint64_t pair = pair0 + w;
         const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
         dedup_pair((uint32_t)w + 1u, b, e, ws, Q.lw[qi], Q.len[qi], L.len[si], ucut, hits, ub, flags, bb, bt, cells + b);
+    }
+}
+
+// The same replay, a bucket a thread.  The hash's buckets are independent (a chain holds one bucket's
+// cells, and a stale cell is recycled only inside its chain, diag_hash.rs:51-110), so the hits sorted
+// by (pair, bucket), in scan order within, are as many separate replays as there are runs of one key.
+// Bound: the latency of the longest run's chain of steps, where k_dedup's is that of the pair with
+// the most hits (a 2.1 Mb contig against 50 consensi: 215,000 hits a pair, 420 a bucket); for many
+// pairs with few hits it is the traffic of the sort.
+__device__ __forceinline__ void diag_of(const SeedHit h, uint32_t qlen, uint32_t slen, uint32_t lw, int32_t& diag,
+                                        uint32_t& key) {
+    const uint32_t qo = h.qs & 0x7fffffffu, so = h.s;
+    if (!(h.qs >> 31)) {
+        diag = (int32_t)(so - qo);
+        key = so;
+    } else {
+        diag = (int32_t)(slen - 2u * qlen - 1u + (qo - so));
+        key = slen - so - lw;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_bucket_keys(DevLib L, DevQueries Q, uint64_t pair0, uint64_t n,
+                                                     const SeedHit* __restrict__ hits,
+                                                     const uint32_t* __restrict__ hit_pair, uint32_t* __restrict__ keys,
+                                                     uint32_t* __restrict__ vals) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t pair = hit_pair[i], qi = pair / L.n, si = pair % L.n;
+        int32_t diag;
+        uint32_t key;
+        diag_of(hits[i], Q.len[qi], L.len[si], (uint32_t)Q.lw[qi], diag, key);
+        keys[i] = (uint32_t)(pair - pair0) * 512u + diag_bucket(diag);
+        vals[i] = (uint32_t)i;
+    }
+}
+
+// The sorted hits' diagonals and hash keys, and, with `leaders`, which hits of a dense pair range are
+// extended ahead of the replay (bit 31 of vals): all but those close behind another hit of their
+// diagonal.  A hit on a long identical diagonal is then dropped, or extended in the replay, instead of
+// walking the diagonal's whole length once for every hit on it.
+constexpr uint32_t LEAD_GAP = 64, LEAD_BACK = 4, LEAD = 0x80000000u;
+__global__ void __launch_bounds__(256) k_bucket_gather(DevLib L, DevQueries Q, uint64_t pair0, uint64_t n,
+                                                       const uint32_t* __restrict__ keys,
+                                                       const uint32_t* __restrict__ vals,
+                                                       const SeedHit* __restrict__ hits, int32_t* __restrict__ diags,
+                                                       uint32_t* __restrict__ hash_keys) {
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t pair = pair0 + keys[k] / 512u;
+        const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
+        diag_of(hits[vals[k]], Q.len[qi], L.len[si], (uint32_t)Q.lw[qi], diags[k], hash_keys[k]);
+    }
+}
+__global__ void __launch_bounds__(256) k_bucket_leaders(uint64_t n, const uint32_t* __restrict__ keys,
+                                                        const int32_t* __restrict__ diags,
+                                                        const uint32_t* __restrict__ hash_keys,
+                                                        uint32_t* __restrict__ vals) {
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t run = keys[k], key = hash_keys[k];
+        const int32_t diag = diags[k];
+        bool lead = true;
+#pragma unroll
+        for (uint32_t b = 1; b <= LEAD_BACK; ++b)
+            if (b <= k && keys[k - b] == run && diags[k - b] == diag && key - hash_keys[k - b] <= LEAD_GAP) lead = false;
+        if (lead) vals[k] |= LEAD;
+    }
+}
+
+// Thread k replays the run that starts at sorted hit k; its chain, oldest cell first, is
+// cells[k ..] with the newest cell in registers.  The hits come in batches whose loads go out
+// together (a run of thousands of hits, a query against itself, waits for one batch after another).
+// SOME: only the hits with bit 31 have a box; an admitted one without is extended here.
+constexpr int REPLAY_BATCH = 8;
+template <bool SOME>
+__global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, const DevParams* __restrict__ P, int32_t ws,
+                                                      int32_t ucut, uint64_t pair0, uint64_t n,
+                                                      const uint32_t* __restrict__ keys,
+                                                      const uint32_t* __restrict__ vals,
+                                                      const int32_t* __restrict__ diags,
+                                                      const uint32_t* __restrict__ hash_keys,
+                                                      const SeedHit* __restrict__ hits, UngBox* __restrict__ ub,
+                                                      uint8_t* __restrict__ flags, DiagCell* __restrict__ cells) {
+    __shared__ int32_t mat[SOME ? 256 : 1];
+    if (SOME) {
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) mat[i] = P->matrix[i];
+        __syncthreads();
+    }
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uint32_t run = keys[k];
+    if (k > 0 && keys[k - 1] == run) return;
+    const int32_t window = 1 - ws;
+    DiagCell* pool = cells + k;
+    DiagCell head{0, 0, 0};
+    uint32_t m = 0;  // cells, the head included; the others are pool[0 .. m - 2]
+    bool more = true;
+    for (uint64_t j = k; more; j += REPLAY_BATCH) {
+        uint32_t bi[REPLAY_BATCH], bkey[REPLAY_BATCH], bstore[REPLAY_BATCH];
+        int32_t bdiag[REPLAY_BATCH], bscore[REPLAY_BATCH];
+        int cnt = 0;
+#pragma unroll
+        for (int b = 0; b < REPLAY_BATCH; ++b) {
+            const bool in = cnt == b && j + b < n && keys[j + b] == run;
+            cnt += in;
+            bi[b] = in ? vals[j + b] : 0;
+            bdiag[b] = in ? diags[j + b] : 0;
+            bkey[b] = in ? hash_keys[j + b] : 0;
+        }
+        more = cnt == REPLAY_BATCH;
+#pragma unroll
+        for (int b = 0; b < REPLAY_BATCH; ++b)
+            if (b < cnt && (!SOME || bi[b] & LEAD)) {
+                bstore[b] = ub[bi[b] & ~LEAD].store;
+                bscore[b] = ub[bi[b] & ~LEAD].score;
+            }
+#pragma unroll
+        for (int b = 0; b < REPLAY_BATCH; ++b) {
+            if (b >= cnt) break;
+            const uint32_t i = bi[b] & ~LEAD, key = bkey[b];
+            const int32_t diag = bdiag[b];
+            uint32_t last = 0;
+            bool known = m > 0 && head.diag == diag;
+            if (known) last = head.level;
+            for (uint32_t c = m; !known && c > 1; --c)
+                if (pool[c - 2].diag == diag) {
+                    last = pool[c - 2].level;
+                    known = true;
+                }
+            if (key < last) {
+                flags[i] = 0;
+                continue;
+            }
+            if (SOME && !(bi[b] & LEAD)) {
+                const uint64_t pair = pair0 + run / 512u;
+                const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
+                const uint32_t qlen = Q.len[qi], slen = L.len[si];
+                const SeedHit h = hits[i];
+                UngBox u;
+                uint32_t a, e, c, d;
+                UngWalk walk;
+                const int32_t qo = (int32_t)(h.qs & 0x7fffffffu), so = (int32_t)h.s;
+                const uint8_t* sp = L.plus + L.plus_off[si];
+                if (!(h.qs >> 31)) walk.start(Q.q + Q.off[qi], sp, (int32_t)qlen, (int32_t)slen, qo, so, P->xdrop_ungap);
+                else walk.start(Q.qrc + Q.off[qi], sp, (int32_t)qlen, (int32_t)slen, (int32_t)qlen - 1 - qo,
+                                (int32_t)slen - 1 - so, P->xdrop_ungap);
+                while (walk.step(mat) != 2) {
+                }
+                walk.result(u.score, a, e, c, d);
+                if (!(h.qs >> 31)) {
+                    u.q_start = a; u.q_end = e; u.s_start = c; u.s_end = d;
+                    u.store = u.score >= ucut ? d : h.s + (uint32_t)ws;
+                } else {
+                    u.q_start = qlen - e; u.q_end = qlen - a; u.s_start = slen - d; u.s_end = slen - c;
+                    u.store = u.score >= ucut ? d : key + (uint32_t)ws;
+                }
+                ub[i] = u;
+                bstore[b] = u.store;
+                bscore[b] = u.score;
+            }
+            flags[i] = bscore[b] >= ucut ? 3 : 1;
+            if (m > 0 && (head.diag == diag || (int32_t)(key - head.level) > window)) {
+                head.diag = diag;
+                head.level = bstore[b];
+                continue;
+            }
+            bool done = false;
+            for (uint32_t c = m; !done && c > 1; --c) {
+                DiagCell& cl = pool[c - 2];
+                if (cl.diag == diag || (int32_t)(key - cl.level) > window) {
+                    cl.diag = diag;
+                    cl.level = bstore[b];
+                    done = true;
+                }
+            }
+            if (!done) {
+                if (m > 0) pool[m - 1] = head;
+                head = DiagCell{diag, bstore[b], 0};
+                ++m;
+            }
+        }
     }
 }
 
@@ -2257,18 +2441,20 @@ cudaError_t launch_scan_gather(uint64_t pair0, uint64_t n_pairs, const uint32_t*
 
 cudaError_t launch_ungapped(const DevLib& L, const DevQueries& Q, const DevParams* P, int32_t ucut, uint64_t n,
                             const SeedHit* hits, const uint32_t* hit_pair, UngBox* out, int sms, cudaStream_t st,
-                            unsigned long long* queue, int blocks_per_sm) {
+                            unsigned long long* queue, int blocks_per_sm, const uint32_t* list,
+                            const unsigned int* n_list) {
     if (!n) return cudaSuccess;
     const int block = 256;
     if (!queue) {  // plain: one hit per thread
         k_ungapped<false><<<(unsigned)((n + block - 1) / block), block, 0, st>>>(L, Q, P, ucut, n, hits, hit_pair,
-                                                                                 out, nullptr);
+                                                                                 out, nullptr, nullptr, nullptr);
         return cudaGetLastError();
     }
     cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     const int bps = blocks_per_sm < 1 ? 1 : blocks_per_sm > 8 ? 8 : blocks_per_sm;
-    k_ungapped<true><<<grid_for(n, block, bps, sms), block, 0, st>>>(L, Q, P, ucut, n, hits, hit_pair, out, queue);
+    k_ungapped<true><<<grid_for(n, block, bps, sms), block, 0, st>>>(L, Q, P, ucut, n, hits, hit_pair, out, queue,
+                                                                     list, n_list);
     return cudaGetLastError();
 }
 
@@ -2282,6 +2468,63 @@ cudaError_t launch_dedup(const DevLib& L, const DevQueries& Q, int32_t ws, int32
     const uint64_t cap = dedup_threads(sms) / block;
     const int grid = (int)(want < cap ? (want ? want : 1) : cap);
     k_dedup<<<grid, block, 0, st>>>(L, Q, ws, ucut, pair0, n_pairs, offs, hits, ub, flags, scratch, (DiagCell*)cells);
+    return cudaGetLastError();
+}
+
+// keys and values before and after the sort, the extended hits and their count
+size_t bucket_dedup_bytes(uint64_t n) { return 5 * ((n * 4 + 255) & ~255ull) + 256; }
+// pairs that a sort key has room for beside the bucket, hits that a value has beside its bit
+bool bucket_dedup_fits(uint64_t n_pairs, uint64_t n) { return n_pairs <= (1ull << 23) && n < LEAD; }
+
+struct IsLead {
+    __host__ __device__ bool operator()(const uint32_t& v) const { return v & LEAD; }
+};
+
+cudaError_t launch_bucket_dedup(const DevLib& L, const DevQueries& Q, const DevParams* P, int32_t ws, int32_t ucut,
+                                uint64_t pair0, uint64_t n_pairs, uint64_t n, const SeedHit* hits,
+                                const uint32_t* hit_pair, UngBox* ub, uint8_t* flags, void* cells,
+                                unsigned long long* queue, int blocks_per_sm, bool leaders, void* buf, void* temp,
+                                size_t& temp_bytes, int sms, cudaStream_t st) {
+    const size_t part = (n * 4 + 255) & ~255ull;
+    uint32_t* keys = (uint32_t*)buf;  // free after the sort: then the sorted hits' diagonals and hash keys
+    uint32_t* vals = (uint32_t*)((char*)buf + part);
+    uint32_t* keys2 = (uint32_t*)((char*)buf + 2 * part);
+    uint32_t* vals2 = (uint32_t*)((char*)buf + 3 * part);
+    uint32_t* lead = (uint32_t*)((char*)buf + 4 * part);
+    unsigned int* n_lead = (unsigned int*)((char*)buf + 5 * part);
+    int bits = 9;
+    while (bits < 32 && (n_pairs << 9) > (1ull << bits)) ++bits;
+    if (!temp) {
+        size_t t_sort = 0, t_sel = 0;
+        cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, t_sort, keys, keys2, vals, vals2, (int64_t)n, 0, bits, st);
+        if (e == cudaSuccess && leaders)
+            e = cub::DeviceSelect::If(nullptr, t_sel, vals2, lead, n_lead, (int64_t)n, IsLead{}, st);
+        temp_bytes = std::max(t_sort, t_sel);
+        return e;
+    }
+    if (!n) return cudaSuccess;
+    const int grid = grid_for(n, 256, 8, sms);
+    k_bucket_keys<<<grid, 256, 0, st>>>(L, Q, pair0, n, hits, hit_pair, keys, vals);
+    size_t tb = temp_bytes;
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys2, vals, vals2, (int64_t)n, 0, bits, st);
+    if (e != cudaSuccess) return e;
+    int32_t* diags = (int32_t*)keys;
+    uint32_t* hash_keys = vals;
+    k_bucket_gather<<<grid, 256, 0, st>>>(L, Q, pair0, n, keys2, vals2, hits, diags, hash_keys);
+    const unsigned runs = (unsigned)((n + 127) / 128);
+    if (leaders) {
+        k_bucket_leaders<<<grid, 256, 0, st>>>(n, keys2, diags, hash_keys, vals2);
+        tb = temp_bytes;
+        e = cub::DeviceSelect::If(temp, tb, vals2, lead, n_lead, (int64_t)n, IsLead{}, st);
+        if (e != cudaSuccess) return e;
+        e = launch_ungapped(L, Q, P, ucut, n, hits, hit_pair, ub, sms, st, queue, blocks_per_sm, lead, n_lead);
+        if (e != cudaSuccess) return e;
+        k_bucket_dedup<true><<<runs, 128, 0, st>>>(L, Q, P, ws, ucut, pair0, n, keys2, vals2, diags, hash_keys, hits, ub,
+                                                   flags, (DiagCell*)cells);
+    } else {
+        k_bucket_dedup<false><<<runs, 128, 0, st>>>(L, Q, P, ws, ucut, pair0, n, keys2, vals2, diags, hash_keys, hits, ub,
+                                                    flags, (DiagCell*)cells);
+    }
     return cudaGetLastError();
 }
 

@@ -25,7 +25,8 @@ cudaError_t launch_scan_gather(uint64_t pair0, uint64_t n_pairs, const uint32_t*
 // queue: 8 bytes of device scratch (the hit queue counter; zeroed here)
 cudaError_t launch_ungapped(const DevLib& L, const DevQueries& Q, const DevParams* P, int32_t ucut, uint64_t n,
                             const SeedHit* hits, const uint32_t* hit_pair, UngBox* out, int sms, cudaStream_t st,
-                            unsigned long long* queue, int blocks_per_sm = 8);
+                            unsigned long long* queue, int blocks_per_sm = 8, const uint32_t* list = nullptr,
+                            const unsigned int* n_list = nullptr);
 uint64_t dedup_threads(int sms);
 // Bucket-parallel diagonal dedup that extends only the hits the hash admits (one warp per pair):
 // flags and boxes as launch_ungapped + launch_dedup give them.
@@ -39,6 +40,16 @@ size_t diag_cell_bytes();
 cudaError_t launch_dedup(const DevLib& L, const DevQueries& Q, int32_t ws, int32_t ucut, uint64_t pair0,
                          uint64_t n_pairs, const uint64_t* offs, const SeedHit* hits, const UngBox* ub, uint8_t* flags,
                          uint32_t* scratch, void* cells, int sms, cudaStream_t st);
+// The dedup by (pair, bucket): of launch_ungapped's boxes, or, with `leaders`, extending hits itself
+// (queue and blocks_per_sm as launch_ungapped's).  buf holds bucket_dedup_bytes(n); with a null temp only temp_bytes is set.
+// The range has to pass bucket_dedup_fits.
+size_t bucket_dedup_bytes(uint64_t n);
+bool bucket_dedup_fits(uint64_t n_pairs, uint64_t n);
+cudaError_t launch_bucket_dedup(const DevLib& L, const DevQueries& Q, const DevParams* P, int32_t ws, int32_t ucut,
+                                uint64_t pair0, uint64_t n_pairs, uint64_t n, const SeedHit* hits,
+                                const uint32_t* hit_pair, UngBox* ub, uint8_t* flags, void* cells,
+                                unsigned long long* queue, int blocks_per_sm, bool leaders, void* buf, void* temp,
+                                size_t& temp_bytes, int sms, cudaStream_t st);
 cudaError_t launch_prelim(const DevLib& L, const DevQueries& Q, const DevParams* P, uint64_t n, const uint32_t* list,
                           const uint32_t* idx, const SeedHit* hits, const uint32_t* hit_pair, const UngBox* ub,
                           PrelimOut* out, uint32_t* wide, unsigned int* n_wide, unsigned long long* cells, int sms,
