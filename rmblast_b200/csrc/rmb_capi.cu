@@ -229,6 +229,7 @@ struct rmb_ctx {
     bool prelim_stream = false;  // thread-per-extension prelim kernel (else the warp kernel)
     bool prelim_pack = false;    // within it, the packed-row kernels
     bool prelim_dual = false;    // with k_prelim_dual before k_prelim_pack
+    bool tb_pack = false;        // the traceback with the band in registers
     rmb_tune tune = default_tune();  // launch knobs of the batched pipeline (rmb_tune_set / rmb_autotune)
     KaBlock ka;                  // E-value statistics (lambda <= 0: none)
     // DUST: the segments' units, converted bases, marks and per-query words; the bases that N draws;
@@ -1399,14 +1400,26 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                     std::stable_sort(todo.begin(), todo.end(), [&](uint32_t x, uint32_t y) { return box(x) > box(y); });
                 uint64_t trace_cap = 1ull << 20;
                 uint32_t ops_cap = 1024;
+                // the packed kernel first; the prelims that its window does not fit go to the byte-trace one
+                bool packed = C.tb_pack;
+                uint32_t trace_rows = std::min<uint64_t>(1u << 14, (uint64_t)qmax + 2);
+                std::vector<uint32_t> wide;
                 int rounds = 0;
-                while (!todo.empty()) {
+                while (!todo.empty() || !wide.empty()) {
+                    if (todo.empty()) {
+                        todo.swap(wide);
+                        packed = false;
+                        ops_cap = 1024;
+                        rounds = 0;
+                    }
                     if (++rounds > 12) throw Fail(RMB_ENOMEM, "traceback scratch kept overflowing");
                     std::vector<TbIn> chunk_in(todo.size());
                     for (size_t i = 0; i < todo.size(); ++i) chunk_in[i] = tin[todo[i]];
                     const uint64_t band_cells = (uint64_t)C.max_slen + 2;
                     const uint32_t rows_cap = qmax + 2;
-                    const uint64_t per_thread = ((band_cells * 8 + (uint64_t)rows_cap * 8 + trace_cap) + 255) & ~255ull;
+                    const uint64_t per_thread =
+                        packed ? traceback_pack_bytes(trace_rows)
+                               : ((band_cells * 8 + (uint64_t)rows_cap * 8 + trace_cap) + 255) & ~255ull;
                     const uint64_t budget = 8ull << 30;
                     // one warp per scratch slot (two items, the left and the right extension, per
                     // prelim), blocks of 8 warps
@@ -1414,6 +1427,8 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                     const bool whole = C.p.pipeline == 1;
                     uint32_t threads = (uint32_t)std::min<uint64_t>((whole ? 1 : 2) * todo.size(),
                                                                     std::max<uint64_t>(8, budget / per_thread));
+                    // (no more warps than the packed kernel keeps resident)
+                    if (packed) threads = std::min<uint32_t>(threads, (uint32_t)C.sms * 32);
                     threads = (threads + 7) / 8 * 8;
                     upload(W.tb_in, chunk_in, st);
                     W.tb_out.ensure(todo.size() * sizeof(TbOut));
@@ -1425,11 +1440,16 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                     EvTimer et;
                     et.start(st);
                     ctr.launches += 2;
-                    CK(launch_traceback(C.L, Q, C.d_params.as<DevParams>(), (uint32_t)todo.size(), W.tb_in.as<TbIn>(),
-                                        W.tb_out.as<TbOut>(), W.tb_half.as<TbHalf>(), W.tb_ops.as<uint32_t>(), ops_cap,
-                                        W.tb_scratch.as<uint8_t>(),
-                                        per_thread, band_cells, rows_cap, threads, W.tb_cells.as<unsigned long long>(),
-                                        whole, st));
+                    if (packed)
+                        CK(launch_traceback_pack(C.L, Q, C.d_params.as<DevParams>(), (uint32_t)todo.size(),
+                                                 W.tb_in.as<TbIn>(), W.tb_out.as<TbOut>(), W.tb_half.as<TbHalf>(),
+                                                 W.tb_ops.as<uint32_t>(), ops_cap, W.tb_scratch.as<uint8_t>(), trace_rows,
+                                                 threads, W.tb_cells.as<unsigned long long>(), whole, st));
+                    else
+                        CK(launch_traceback(C.L, Q, C.d_params.as<DevParams>(), (uint32_t)todo.size(),
+                                            W.tb_in.as<TbIn>(), W.tb_out.as<TbOut>(), W.tb_half.as<TbHalf>(),
+                                            W.tb_ops.as<uint32_t>(), ops_cap, W.tb_scratch.as<uint8_t>(), per_thread,
+                                            band_cells, rows_cap, threads, W.tb_cells.as<unsigned long long>(), whole, st));
                     et.stop(st);
                     std::vector<TbOut> to(todo.size());
                     CK(cudaMemcpyAsync(to.data(), W.tb_out.p, to.size() * sizeof(TbOut), cudaMemcpyDeviceToHost, st));
@@ -1439,7 +1459,7 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                     // only the ops of the finished items come back, packed
                     std::vector<uint64_t> ooff(todo.size() + 1, 0);
                     for (size_t i = 0; i < todo.size(); ++i)
-                        ooff[i + 1] = ooff[i] + (to[i].status == 2 ? 0 : to[i].n_ops);
+                        ooff[i + 1] = ooff[i] + (to[i].status > 1 ? 0 : to[i].n_ops);
                     std::vector<uint32_t> ops(ooff.back());
                     if (!ops.empty()) {
                         upload(W.tb_ooff, ooff, st);
@@ -1456,6 +1476,7 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                     for (size_t i = 0; i < todo.size(); ++i) {
                         const TbOut& o = to[i];
                         if (o.status == 2) { again.push_back(todo[i]); continue; }
+                        if (o.status == 4) { wide.push_back(todo[i]); continue; }
                         if (o.status == 3) throw Fail(RMB_ECUDA, "traceback walk did not reach the origin");
                         TbResult& r = tres[todo[i]];
                         r.status = o.status;
@@ -1469,12 +1490,10 @@ bool traceback_2b(rmb_ctx& C, Work& W, const DevQueries& Q, const uint32_t* hqle
                         raw_n[todo[i]] = o.n_ops;
                     }
                     rounds_ops.push_back(std::move(ops));
-                    if (again.size() == todo.size()) {  // nothing finished: grow the caps
+                    if (!again.empty()) {  // grow the caps
                         trace_cap *= 4;
                         ops_cap *= 4;
-                    } else if (!again.empty()) {
-                        trace_cap *= 4;
-                        ops_cap *= 4;
+                        trace_rows = (uint32_t)std::min<uint64_t>(4ull * trace_rows, (uint64_t)qmax + 2);
                     }
                     ctr.tb_cells += cells;
                     todo.swap(again);
@@ -1634,6 +1653,7 @@ int rmb_ctx_create(const rmb_params* params, const int32_t scores[256], const do
         for (int i = 0; i < 256; ++i) dp.matrix[i] = scores[i];
         C->prelim_stream = p.kernels == 0 && prelim_stream_eligible(dp.matrix, p.gap_open, p.gap_extend, p.xdrop_gap);
         C->prelim_pack = C->prelim_stream && prelim_pack_eligible(dp.matrix, p.gap_open, p.gap_extend, p.xdrop_gap);
+        C->tb_pack = traceback_pack_eligible(dp.matrix, p.gap_open, p.gap_extend, p.xdrop_gap_final);
         C->prelim_dual = C->prelim_pack && prelim_dual_pays(dp.matrix, p.word_size, dp.gapped_cutoff);
         if (p.ka_lambda > 0.0) {
             if (!(p.ka_k > 0.0) || !(p.ka_h > 0.0) || !(p.ka_alpha > 0.0))

@@ -32,6 +32,7 @@
 #include <cub/device/device_select.cuh>
 #include <thrust/iterator/counting_iterator.h>
 #include "rmb_sched.cuh"
+#include "rmb_traceback_pack.cuh"
 #include "rmb_ungapped.cuh"
 
 namespace rmb {
@@ -2298,21 +2299,80 @@ __global__ void __launch_bounds__(256) k_traceback_warp(DevLib L, DevQueries Q, 
     if (lane == 0 && cells) atomicAdd(cells_total, (unsigned long long)cells);
 }
 
+// k_traceback_warp's items with the band in registers (rmb_traceback_pack.cuh); `per_warp` bytes of scratch
+// a warp hold rows_cap rows of trace and their window positions.
+__global__ void __launch_bounds__(128) k_traceback_pack(DevLib L, DevQueries Q, const DevParams* __restrict__ P,
+                                                         uint32_t n, const TbIn* __restrict__ in,
+                                                         TbHalf* __restrict__ half, uint32_t* __restrict__ ops_out,
+                                                         uint32_t ops_cap, uint8_t* __restrict__ scratch,
+                                                         uint64_t per_warp, uint32_t rows_cap, bool whole) {
+    __shared__ TbTable tab;
+    const int32_t go = P->gap_open, ge = P->gap_extend, xdrop = P->xdrop_gap_final;
+    if (threadIdx.x < 16) {
+        uint32_t lo[2] = {0, 0}, hi[2] = {0, 0};
+        for (int c = 0; c < 8; ++c) {
+            int32_t v = c < 4 ? P->matrix[threadIdx.x * 16 + c] : c == 4 ? P->matrix[threadIdx.x * 16 + 14] : TB_SCORE_MIN;
+            v = max(v + 2 * ge, TB_SCORE_MIN);
+            lo[c >> 2] |= ((uint32_t)v & 0xffu) << (8 * (c & 3));
+            hi[c >> 2] |= (((uint32_t)v >> 8) & 0xffu) << (8 * (c & 3));
+        }
+        tab.row[threadIdx.x] = make_uint4(lo[0], lo[1], hi[0], hi[1]);
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t k_first = whole ? 2 * warp : warp, k_stride = whole ? 2 * nwarps : nwarps;
+    uint16_t* trace = (uint16_t*)(scratch + warp * per_warp);
+    int32_t* win = (int32_t*)(trace + (uint64_t)rows_cap * 32);
+    for (uint64_t k0 = k_first; k0 < 2ull * n; k0 += k_stride)
+    for (uint64_t k = k0; k < (whole ? k0 + 2 : k0 + 1); ++k) {
+        const uint64_t t = k >> 1;
+        const bool right = k & 1;
+        const TbIn h = in[t];
+        const uint32_t qi = h.pair / L.n, si = h.pair % L.n;
+        const uint32_t qa = Q.len[qi], sa = L.len[si];
+        const bool plus = h.strand == 0;
+        const uint8_t* qfwd = Q.q + Q.off[qi] + 1;
+        const uint8_t* sfs = (plus ? L.align : L.align_rc) + L.plus_off[si] + 1;
+        uint32_t nq = 0, ns = 0;
+        if (lane == 0) improve_seed(qfwd, qa, sfs, sa, h.q_seed, h.s_seed, h.q_start, h.q_end, h.s_start, h.s_end, !plus, nq, ns);
+        nq = __shfl_sync(0xffffffffu, nq, 0);
+        ns = __shfl_sync(0xffffffffu, ns, 0);
+        const uint32_t tq = plus ? nq : qa - 1 - nq, ts = plus ? ns : sa - 1 - ns;
+        const uint8_t* qs = (plus ? Q.q : Q.qrc) + Q.off[qi] + 1;
+        const uint8_t* ss = L.align + L.plus_off[si] + 1;
+        // left: residues tq, ts downwards; right: tq + 1, ts + 1 upwards
+        const int32_t m = right ? (int32_t)qa - (int32_t)tq - 1 : (int32_t)tq + 1;
+        const int32_t nc = right ? (int32_t)sa - (int32_t)ts - 1 : (int32_t)ts + 1;
+        int32_t sc = 0;
+        uint32_t a = 0, b = 0, nops = 0;
+        uint64_t cells = 0;
+        const int st = tb_pack_extend(qs + tq + right, ss + ts + right, right ? 1 : -1, m, nc, go, ge, xdrop, tab, trace, win,
+                                      rows_cap, sc, a, b, ops_out + k * (uint64_t)ops_cap, ops_cap, nops, cells);
+        if (lane == 0) half[k] = TbHalf{st, sc, a, b, nops, (uint32_t)min(cells, (uint64_t)0xffffffffu), tq, ts};
+        __syncwarp();  // the walk's reads before the next extension's writes
+    }
+}
+
 // One prelim per thread: its two extensions' scripts merged (the right one reversed after the
 // left one, runs of one op joined), the end gaps pruned, and the box and score of the whole
 // alignment (engine.rs:2953-3039).  The merged script goes to the left item's ops slot.
 __global__ void k_traceback_join(const DevParams* __restrict__ P, uint32_t n, const TbHalf* __restrict__ half,
-                                 uint32_t* __restrict__ ops_out, uint32_t ops_cap, TbOut* __restrict__ out) {
+                                 uint32_t* __restrict__ ops_out, uint32_t ops_cap, TbOut* __restrict__ out,
+                                 unsigned long long* __restrict__ cells_total) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const TbHalf lh = half[2 * t], rh = half[2 * t + 1];
     TbOut o{0, 0, 0, 0, 0, 0, 0, 0};
     if (lh.status != 0 || rh.status != 0) {
-        o.status = lh.status == 3 || rh.status == 3 ? 3 : 2;
+        o.status = lh.status == 3 || rh.status == 3 ? 3 : lh.status == TB_WIDE || rh.status == TB_WIDE ? TB_WIDE : 2;
         o.need = max(lh.status ? lh.need : 0u, rh.status ? rh.need : 0u);
         out[t] = o;
         return;
     }
+    // k_traceback_pack's cells, of the prelims that it finishes (cells_total null: counted by the kernel)
+    if (cells_total && lh.need + rh.need) atomicAdd(cells_total, (unsigned long long)lh.need + rh.need);
     uint32_t* ops = ops_out + 2 * t * (uint64_t)ops_cap;
     const uint32_t* rops = ops_out + (2 * t + 1) * (uint64_t)ops_cap;
     const uint32_t nl = lh.n_ops, nr = rh.n_ops;
@@ -2386,7 +2446,7 @@ __global__ void __launch_bounds__(256) k_gather_ops(uint32_t n, const uint32_t* 
     const int lane = threadIdx.x & 31;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
-        if (out[i].status == 2) continue;
+        if (out[i].status > 1) continue;
         const uint32_t c = out[i].n_ops;
         for (uint32_t k = lane; k < c; k += 32) dst[off[i] + k] = ops[(uint64_t)i * ops_cap + k];
     }
@@ -2900,6 +2960,32 @@ cudaError_t launch_prelim_wide(const DevLib& L, const DevQueries& Q, const DevPa
     return cudaGetLastError();
 }
 
+bool traceback_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop) {
+    // the initial row right of the pivot's diagonal, and 16-bit values: best + origin up to PACK_REBASE
+    // and a row's gain, the diagonals' decay over the window on top
+    const int32_t goe = gap_open + gap_extend, xmax = std::max(xdrop, goe);
+    if (gap_extend < 1 || gap_extend > 40 || gap_open < 0 || xmax > 4000) return false;
+    if ((xmax - goe) / gap_extend + 1 + TB_K >= TB_W - 1) return false;
+    for (int i = 0; i < 256; ++i)
+        if (matrix256[i] > 2000) return false;
+    return true;
+}
+
+uint64_t traceback_pack_bytes(uint32_t rows_cap) { return ((uint64_t)rows_cap * TB_ROW_BYTES + 255) & ~255ull; }
+
+cudaError_t launch_traceback_pack(const DevLib& L, const DevQueries& Q, const DevParams* P, uint32_t n, const TbIn* in,
+                                  TbOut* out, TbHalf* half, uint32_t* ops, uint32_t ops_cap, uint8_t* scratch,
+                                  uint32_t rows_cap, uint32_t warps, unsigned long long* cells, bool whole,
+                                  cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    k_traceback_pack<<<(warps + 3) / 4, 128, 0, st>>>(L, Q, P, n, in, half, ops, ops_cap, scratch,
+                                                      traceback_pack_bytes(rows_cap), rows_cap, whole);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_traceback_join<<<(n + 127) / 128, 128, 0, st>>>(P, n, half, ops, ops_cap, out, cells);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_traceback(const DevLib& L, const DevQueries& Q, const DevParams* P, uint32_t n, const TbIn* in,
                              TbOut* out, TbHalf* half, uint32_t* ops, uint32_t ops_cap, uint8_t* scratch,
                              uint64_t per_thread, uint64_t band_cells, uint32_t rows_cap, uint32_t threads,
@@ -2914,7 +3000,7 @@ cudaError_t launch_traceback(const DevLib& L, const DevQueries& Q, const DevPara
                                              rows_cap, cells, whole);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_traceback_join<<<(n + 127) / 128, 128, 0, st>>>(P, n, half, ops, ops_cap, out);
+    k_traceback_join<<<(n + 127) / 128, 128, 0, st>>>(P, n, half, ops, ops_cap, out, nullptr);
     return cudaGetLastError();
 }
 
