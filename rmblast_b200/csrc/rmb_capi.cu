@@ -162,7 +162,8 @@ struct Work {
     DBuf pv, pv_off, cs, cs_off, cq, cq_off, pos_off, lut_keys, lut_vals, lut_keys2, lut_vals2, lut_counts;
     DBuf counts, offs, hits, hit_pair, ub, flags, dd_scratch, dd_cells, ung_idx, n_sel, po, wide, wide2, dres, geo,
         n_wide, band, sel, surv, cells, fails, temp, tb_in, tb_out, tb_ops, tb_scratch, stage, stage_start, stage_over,
-        tb_ooff, tb_ops2, ung_queue, dd_units, tb_half, tb_cells, pack_list, pack_ctl;
+        tb_ooff, tb_ops2, ung_queue, dd_units, tb_half, tb_cells, pack_list, pack_ctl, unit_counts, unit_offs,
+        seg_first, seg_subject;
     DBuf sched_pred, sched_order, sched_scratch, sched_feat, sched_cells;
     // the device chain as a CUDA graph (chain_graph): its executable, its timing events and the
     // pinned block its counts come back in
@@ -181,7 +182,7 @@ struct Work {
                        &lut_vals2, &lut_counts, &counts, &offs, &hits, &hit_pair, &ub, &flags, &dd_scratch, &dd_cells,
                        &ung_idx, &n_sel, &po, &wide, &wide2, &dres, &geo, &n_wide, &band, &sel, &surv, &cells, &fails,
                        &temp, &tb_in, &tb_out, &tb_ops, &tb_scratch, &stage, &stage_start, &stage_over, &tb_ooff,
-                       &tb_ops2, &ung_queue, &dd_units, &tb_half, &tb_cells, &pack_list, &pack_ctl, &sched_pred, &sched_order, &sched_scratch, &sched_feat, &sched_cells};
+                       &tb_ops2, &ung_queue, &dd_units, &tb_half, &tb_cells, &pack_list, &pack_ctl, &unit_counts, &unit_offs, &seg_first, &seg_subject, &sched_pred, &sched_order, &sched_scratch, &sched_feat, &sched_cells};
         for (DBuf* b : all) b->release();
         if (st) cudaStreamDestroy(st);
         if (st2) cudaStreamDestroy(st2);
@@ -839,11 +840,42 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
         // pair order (pair ids are local to the sub-batch)
         t0 = std::chrono::steady_clock::now();
         const uint64_t npairs = (uint64_t)nb * ns;
+        // the scan's units: whole pairs, or stretches of them where the pairs are few (batched pipeline)
+        std::vector<uint32_t> seg_first;
+        ScanUnits units;
+        if (P.pipeline != 1) {
+            double density = 0;  // words of the densest query a scan position meets by chance
+            uint32_t step = UINT32_MAX;
+            for (uint32_t i = 0; i < nb; ++i) {
+                density = std::max(density, 2.0 * hqlen[i] / (double)(1ull << (2 * hlw[i])));
+                step = std::min(step, (uint32_t)(P.word_size - hlw[i] + 1));
+            }
+            seg_first = scan_segments(nb, C.slen, step, density, C.sms);
+        }
+        uint64_t nunits = npairs;
+        if (!seg_first.empty()) {
+            std::vector<uint32_t> subject(seg_first.back());
+            for (uint32_t i = 0; i < ns; ++i)
+                std::fill(subject.begin() + seg_first[i], subject.begin() + seg_first[i + 1], i);
+            upload(W.seg_first, seg_first, st);
+            upload(W.seg_subject, subject, st);
+            CK(cudaStreamSynchronize(st));  // `subject` goes out of scope
+            units = ScanUnits{W.seg_first.as<uint32_t>(), W.seg_subject.as<uint32_t>(), seg_first.back()};
+            nunits = (uint64_t)nb * seg_first.back();
+            W.unit_counts.ensure((nunits + 1) * 4);
+            W.unit_offs.ensure((nunits + 1) * 8);
+        }
+        auto unit_of = [&](uint64_t pair) {
+            return units.per_query ? pair / ns * units.per_query + seg_first[pair % ns] : pair;
+        };
         W.counts.ensure((npairs + 1) * 4);
         W.offs.ensure((npairs + 1) * 8);
-        W.stage_start.ensure(npairs * 4);
-        W.stage.ensure(scan_stage_entries(npairs, C.sms) * sizeof(SeedHit));
-        W.stage_over.ensure(16);  // the overflow flag and the scan's pair queue
+        // whole pairs: the units' arrays are the pairs'
+        uint32_t* ucounts = (units.per_query ? W.unit_counts : W.counts).as<uint32_t>();
+        uint64_t* uoffs = (units.per_query ? W.unit_offs : W.offs).as<uint64_t>();
+        W.stage_start.ensure(nunits * 4);
+        W.stage.ensure(scan_stage_entries(nunits, C.sms) * sizeof(SeedHit));
+        W.stage_over.ensure(16);  // the overflow flag and the scan's unit queue
         // The batched pipeline feeds the scan's warps pairs from a queue where the sub-batch's
         // query lengths vary (over 2x): a pair's cost then follows its query too, and fixed
         // strides left warps idle (1,000 chunks of 1-200 kb: 54 -> 38 ms a step).  Over queries
@@ -852,15 +884,23 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
         const uint32_t qlo = *std::min_element(hqlen.begin(), hqlen.end());
         const uint32_t qhi = *std::max_element(hqlen.begin(), hqlen.end());
         const bool scan_queue = P.pipeline != 1 && (uint64_t)qhi > 2ull * qlo;
-        CK(cudaMemsetAsync(W.counts.p, 0, (npairs + 1) * 4, st));
+        CK(cudaMemsetAsync(ucounts, 0, (nunits + 1) * 4, st));
         CK(cudaMemsetAsync(W.stage_over.p, 0, 16, st));
         ev.start(st);
-        CK(launch_scan_stage(C.L, Q, P.word_size, npairs, W.counts.as<uint32_t>(), W.stage_start.as<uint32_t>(),
+        CK(launch_scan_stage(C.L, Q, P.word_size, units, nunits, ucounts, W.stage_start.as<uint32_t>(),
                              W.stage.as<SeedHit>(), W.stage_over.as<unsigned int>(), C.sms, st, scan_queue));
         size_t tb = 0;
-        CK(launch_offsets(W.counts.as<uint32_t>(), npairs + 1, W.offs.as<uint64_t>(), nullptr, tb, st));
-        W.temp.ensure(tb);
-        CK(launch_offsets(W.counts.as<uint32_t>(), npairs + 1, W.offs.as<uint64_t>(), W.temp.p, tb, st));
+        // the offsets of n pairs' units from pair pr0 on, and of the pairs
+        auto offsets = [&](uint64_t pr0, uint64_t n) {
+            const uint64_t u0 = unit_of(pr0), u1 = unit_of(pr0 + n);
+            tb = 0;
+            CK(launch_offsets(ucounts + u0, u1 - u0 + 1, uoffs, nullptr, tb, st));
+            W.temp.ensure(tb);
+            CK(launch_offsets(ucounts + u0, u1 - u0 + 1, uoffs, W.temp.p, tb, st));
+            if (units.per_query)
+                CK(launch_pair_offsets(units, ns, pr0, n, uoffs, W.counts.as<uint32_t>(), W.offs.as<uint64_t>(), C.sms, st));
+        };
+        offsets(0, npairs);
         ev.stop(st);
         uint64_t nh = 0;
         unsigned int stage_over = 0;
@@ -891,24 +931,17 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
             const uint64_t npairs = ranges[ri + 1] - pair0;  // the pairs of this range
             const uint64_t nh = ranges.size() > 2 ? hoffs[pair0 + npairs] - hoffs[pair0] : nh_all;
             if (nh >= 0xffffffffull) throw Fail(RMB_ELIMIT, "more than 2^32 word hits in one pair range");
-            if (ranges.size() > 2) {  // offsets local to the range
-                tb = 0;
-                CK(launch_offsets(W.counts.as<uint32_t>() + pair0, npairs + 1, W.offs.as<uint64_t>(), nullptr, tb,
-                                  st));
-                W.temp.ensure(tb);
-                CK(launch_offsets(W.counts.as<uint32_t>() + pair0, npairs + 1, W.offs.as<uint64_t>(), W.temp.p, tb,
-                                  st));
-            }
+            if (ranges.size() > 2) offsets(pair0, npairs);  // local to the range
             W.hits.ensure(nh * sizeof(SeedHit));
             W.hit_pair.ensure(nh * 4);
             ev.start(st);
             if (!stage_over)
-                CK(launch_scan_gather(pair0, npairs, W.counts.as<uint32_t>(), W.offs.as<uint64_t>(),
+                CK(launch_scan_gather(units, ns, unit_of(pair0), unit_of(pair0 + npairs) - unit_of(pair0), ucounts, uoffs,
                                       W.stage_start.as<uint32_t>(), W.stage.as<SeedHit>(), W.hits.as<SeedHit>(),
                                       W.hit_pair.as<uint32_t>(), C.sms, st));
             else  // a warp's stretch of the stage ran out: scan this range again, writing in place
-                CK(launch_scan(true, C.L, Q, P.word_size, pair0, npairs, nullptr, W.offs.as<uint64_t>(),
-                               W.hits.as<SeedHit>(), W.hit_pair.as<uint32_t>(), C.sms, st));
+                CK(launch_scan(C.L, Q, P.word_size, pair0, npairs, W.offs.as<uint64_t>(), W.hits.as<SeedHit>(),
+                               W.hit_pair.as<uint32_t>(), C.sms, st));
             ev.stop(st);
             CK(cudaStreamSynchronize(st));
             ctr.gpu_ms_scan += ev.ms();

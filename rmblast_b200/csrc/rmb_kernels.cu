@@ -56,101 +56,115 @@ struct PairView {
 };
 
 // engine.rs:1118-1149 (plus) and 1187-1218 (minus): exact extension to word_size on the
-// masked query; returns false if the word hit is dropped.
-__device__ __forceinline__ bool exact_extend(const PairView& v, uint32_t q0c, uint32_t p, uint32_t& qs, uint32_t& so) {
+// masked query; returns false if the word hit is dropped.  The two runs of matching bases beside the
+// word, at most ext_needed long, are counted in two plain loops over the whole warp (the sentinels at
+// the sequences' ends stop them), then limited in the strand's order: left first on the plus
+// strand, right first on the minus strand.  Early returns out of the loops are avoided on purpose:
+// with them the warp was seen to reach the caller's vote in two parts (one hit in millions lost).
+__device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint32_t q0c, uint32_t p, uint32_t& qs,
+                                             uint32_t& so) {
     const int64_t c1 = v.qlen + 1;
-    const int64_t lw = v.lw, need = v.ext_needed;
-    if ((int64_t)q0c < c1) {
-        int64_t el = 0, er = 0;
-        if (need > 0) {
-            while (el < need) {
-                int64_t qi = (int64_t)q0c - el - 1, si = (int64_t)p - el - 1;
-                if (qi < 0 || si < 0) break;
-                uint8_t qb = v.qmask[1 + qi], sb = v.splus[1 + si];
-                if (qb >= 4 || sb >= 4 || qb != sb) break;
-                ++el;
-            }
-            while (el + er < need) {
-                int64_t qi = (int64_t)q0c + lw + er, si = (int64_t)p + lw + er;
-                if (qi >= v.qlen || si >= v.slen) break;
-                uint8_t qb = v.qmask[1 + qi], sb = v.splus[1 + si];
-                if (qb >= 4 || sb >= 4 || qb != sb) break;
-                ++er;
-            }
-            if (el + er < need) return false;
+    const bool plus = (int64_t)q0c < c1;
+    // the word's start in the frame that the extension runs in
+    const int64_t q0 = plus ? (int64_t)q0c : v.qlen - ((int64_t)q0c - c1) - v.lw;
+    const int64_t s0 = plus ? (int64_t)p : v.slen - (int64_t)p - v.lw;
+    there = there && q0 >= 0 && s0 >= 0;
+    const int32_t need = v.ext_needed;
+    const uint8_t* q = v.qmask + 1 + q0;
+    const uint8_t* s = (plus ? v.splus : v.src) + 1 + s0;
+    int32_t left = 0, right = 0;
+    bool on = there;
+    for (int32_t i = 0; i < need; ++i) {
+        uint8_t a = 15, b = 0;
+        if (on) {
+            a = q[-1 - i];
+            b = s[-1 - i];
         }
-        qs = (uint32_t)((int64_t)q0c - el);
-        so = (uint32_t)((int64_t)p - el);
-        return true;
+        on = on && a < 4 && a == b;
+        left += on;
     }
-    const int64_t rcq = (int64_t)q0c - c1;
-    const int64_t q0 = v.qlen - rcq - lw, s0 = v.slen - (int64_t)p - lw;
-    if (q0 < 0 || s0 < 0) return false;
-    int64_t el = 0, er = 0;
-    if (need > 0) {
-        while (er < need) {
-            int64_t qi = q0 + lw + er, si = s0 + lw + er;
-            if (qi >= v.qlen || si >= v.slen) break;
-            uint8_t qb = v.qmask[1 + qi], sb = v.src[1 + si];
-            if (qb >= 4 || sb >= 4 || qb != sb) break;
-            ++er;
+    on = there;
+    for (int32_t i = 0; i < need; ++i) {
+        uint8_t a = 15, b = 0;
+        if (on) {
+            a = q[v.lw + i];
+            b = s[v.lw + i];
         }
-        while (el + er < need) {
-            int64_t qi = q0 - el - 1, si = s0 - el - 1;
-            if (qi < 0 || si < 0) break;
-            uint8_t qb = v.qmask[1 + qi], sb = v.src[1 + si];
-            if (qb >= 4 || sb >= 4 || qb != sb) break;
-            ++el;
-        }
-        if (el + er < need) return false;
+        on = on && a < 4 && a == b;
+        right += on;
     }
-    qs = (uint32_t)(q0 + er) | 0x80000000u;
-    so = (uint32_t)(s0 + er);
-    return true;
+    if (plus) right = min(right, need - left);
+    else left = min(left, need - right);
+    qs = plus ? (uint32_t)(q0 - left) : (uint32_t)(q0 + right) | 0x80000000u;
+    so = plus ? (uint32_t)(s0 - left) : (uint32_t)(s0 + right);
+    return there && left + right >= need;
 }
 
-// One warp per (query, subject) pair: the subject's words at the scan stride against the query's
-// lookup table (lookup.rs scan), each word hit extended exactly to word_size.  Hits leave in scan
-// order (subject position, then lookup-cell order).
-//   SCAN_COUNT: per-pair hit counts only.
-//   SCAN_WRITE: hits at the pair's offset in `hits` (offs from the counts).
-//   SCAN_STAGE: counts, and the hits appended to this warp's stretch of `hits` (stage_cap entries
-//               from warp * stage_cap), the pair's first entry in stage_start; if a stretch runs
-//               out, *stage_over is set and the batch takes the SCAN_WRITE pass instead.
-enum { SCAN_COUNT = 0, SCAN_WRITE = 1, SCAN_STAGE = 2 };
+// A scan unit's pair, and which of its stretches it is.
+struct ScanUnit {
+    uint64_t pair;
+    uint32_t seg, n_seg;
+};
+__device__ __forceinline__ ScanUnit scan_unit(const ScanUnits& U, uint32_t n_subjects, uint64_t w) {
+    if (!U.per_query) return ScanUnit{w, 0, 1};
+    const uint64_t q = w / U.per_query;
+    const uint32_t x = (uint32_t)(w % U.per_query), si = U.subject[x], first = U.first[si];
+    return ScanUnit{q * n_subjects + si, x - first, U.first[si + 1] - first};
+}
+__device__ __forceinline__ uint64_t scan_unit_of(const ScanUnits& U, uint32_t n_subjects, uint64_t pair) {
+    return U.per_query ? pair / n_subjects * U.per_query + U.first[pair % n_subjects] : pair;
+}
+
+// One warp per unit, a (query, subject) pair or one of its stretches of scan positions: the
+// subject's words at the scan stride against the query's lookup table (lookup.rs scan), each word hit
+// extended exactly to word_size.  Hits leave in scan order (subject position, then lookup-cell order).
+//   SCAN_WRITE: hits at the pair's offset in `hits` (offs from the counts; whole pairs).
+//   SCAN_STAGE: counts per unit, and the hits appended to this warp's stretch of `hits` (stage_cap
+//               entries from warp * stage_cap), the unit's first entry in stage_start; if a stretch
+//               runs out, *stage_over is set and the batch takes the SCAN_WRITE pass instead.
+// Bound: the latency of a round's dependent loads (subject word, presence bit, cell start, cell entry,
+// query bytes).  So a round takes SCAN_POS positions a lane, their loads side by side, and its cells'
+// entries are spread over the warp as one list, one entry a lane.  Measured (B200) against one position a
+// lane and round: 1,000 contigs against 2,000 consensi (2 M pairs) 31 -> 18 ms, 120 chunks of 60 kb
+// 8.2 -> 3.3, 4,000 sequences at word 14 11.3 -> 8.2; and by stretches of pairs, 100 kb at word 7
+// 5.5 -> 0.1, 2.1 Mb against 2,000 consensi 50 -> 1.
+enum { SCAN_WRITE = 1, SCAN_STAGE = 2 };
+constexpr int SCAN_POS = 4;
+constexpr uint32_t SCAN_ROUND = 32 * SCAN_POS;
 
 template <int MODE>
-__global__ void __launch_bounds__(256) k_scan(DevLib L, DevQueries Q, int32_t ws, uint64_t pair0, uint64_t n_pairs,
-                                               uint32_t* counts, const uint64_t* offs, SeedHit* hits,
+__global__ void __launch_bounds__(256) k_scan(DevLib L, DevQueries Q, int32_t ws, uint64_t pair0, uint64_t n_units,
+                                               ScanUnits U, uint32_t* counts, const uint64_t* offs, SeedHit* hits,
                                                uint32_t* hit_pair, uint32_t* stage_start, uint32_t stage_cap,
-                                               unsigned int* stage_over, unsigned long long* pair_queue) {
-    constexpr bool WRITE = MODE != SCAN_COUNT;
-    // per warp: each lane's first candidate index, lookup-cell start and scan position
-    __shared__ uint32_t s_first[8][32], s_cell[8][32], s_pos[8][32];
+                                               unsigned int* stage_over, unsigned long long* unit_queue) {
+    // per warp: each lane's first candidate, and its positions' cell starts and running counts
+    __shared__ uint32_t s_first[8][32];
+    __shared__ uint32_t s_cell[8][32][SCAN_POS], s_end[8][32][SCAN_POS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const uint32_t stage0 = MODE == SCAN_STAGE ? (uint32_t)warp * stage_cap : 0u;  // this warp's stretch
     uint32_t cursor = 0;                                                            // entries of it used
     bool fits = true;
-    // pairs by warp stride, or, with pair_queue, the next pair off a grid-wide counter as a warp
+    // units by warp stride, or, with unit_queue, the next unit off a grid-wide counter as a warp
     // finishes one (subject lengths vary 100-fold, so fixed strides leave warps idle at the end)
     uint64_t w_next = warp;
-    auto next_pair = [&]() -> uint64_t {
-        if (pair_queue) {
+    auto next_unit = [&]() -> uint64_t {
+        if (unit_queue) {
             unsigned long long x = 0;
-            if (lane == 0) x = atomicAdd(pair_queue, 1ull);
+            if (lane == 0) x = atomicAdd(unit_queue, 1ull);
             return __shfl_sync(0xffffffffu, x, 0);
         }
         const uint64_t r = w_next;
         w_next += nwarps;
         return r;
     };
-    for (uint64_t w = next_pair(); w < n_pairs; w = next_pair()) {
-        const uint64_t pair = pair0 + w;
+    for (uint64_t w = next_unit(); w < n_units; w = next_unit()) {
+        const ScanUnit unit = scan_unit(U, L.n, w);
+        const uint64_t pair = pair0 + unit.pair;
         const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
         const uint32_t qlen = Q.len[qi], slen = L.len[si];
-        uint64_t out = MODE == SCAN_WRITE ? offs[w] : MODE == SCAN_STAGE ? (uint64_t)(stage0 + cursor) : 0;
+        uint64_t out = MODE == SCAN_WRITE ? offs[w] : (uint64_t)(stage0 + cursor);
         uint32_t total = 0;
         if (qlen >= (uint32_t)ws && slen >= (uint32_t)ws) {
             PairView v;
@@ -167,50 +181,70 @@ __global__ void __launch_bounds__(256) k_scan(DevLib L, DevQueries Q, int32_t ws
             const uint32_t* pv = Q.pv + Q.pv_off[qi];
             const uint32_t* cs = Q.cell_start + Q.cs_off[qi];
             const uint32_t* cq = Q.cell_q + Q.cq_off[qi];
-            for (uint32_t k0 = 0; k0 < npos; k0 += 32) {
-                // lane l looks up position k0 + l; its lookup cell's entries b .. b + cnt are
-                // then spread over the warp, one entry a lane, in (position, entry) order
-                const uint32_t k = k0 + lane;
-                uint32_t cnt = 0, b = 0, p = 0;
-                if (k < npos) {
-                    p = k * step;
-                    const uint32_t idx = kmer_at(pk, p, v.lw);
-                    if (__ldg(pv + (idx >> 5)) & (1u << (idx & 31))) {
-                        b = __ldg(cs + idx);
-                        cnt = __ldg(cs + idx + 1) - b;
-                    }
+            const uint32_t rounds = (npos + SCAN_ROUND - 1) / SCAN_ROUND;
+            const uint32_t r_begin = (uint32_t)((uint64_t)rounds * unit.seg / unit.n_seg);
+            const uint32_t r_end = (uint32_t)((uint64_t)rounds * (unit.seg + 1) / unit.n_seg);
+            for (uint32_t r = r_begin; r < r_end; ++r) {
+                // lane l looks up positions k0 .. k0 + SCAN_POS - 1
+                const uint32_t k0 = r * SCAN_ROUND + (uint32_t)lane * SCAN_POS;
+                uint32_t idx[SCAN_POS], cell[SCAN_POS], cnt[SCAN_POS];
+                bool there[SCAN_POS];
+#pragma unroll
+                for (int u = 0; u < SCAN_POS; ++u) {
+                    there[u] = k0 + u < npos;
+                    idx[u] = there[u] ? kmer_at(pk, (k0 + u) * step, v.lw) : 0u;
                 }
-                uint32_t incl = cnt;
+#pragma unroll
+                for (int u = 0; u < SCAN_POS; ++u) there[u] = there[u] && (__ldg(pv + (idx[u] >> 5)) & (1u << (idx[u] & 31)));
+                bool some = false;
+#pragma unroll
+                for (int u = 0; u < SCAN_POS; ++u) some |= there[u];
+                if (!__any_sync(0xffffffffu, some)) continue;
+#pragma unroll
+                for (int u = 0; u < SCAN_POS; ++u) {
+                    cell[u] = there[u] ? __ldg(cs + idx[u]) : 0u;
+                    cnt[u] = there[u] ? __ldg(cs + idx[u] + 1) : 0u;
+                }
+                uint32_t mine = 0;
+#pragma unroll
+                for (int u = 0; u < SCAN_POS; ++u) {
+                    cnt[u] -= cell[u];
+                    mine += cnt[u];
+                    s_cell[wib][lane][u] = cell[u];
+                    s_end[wib][lane][u] = mine;
+                }
+                uint32_t incl = mine;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
                     if (lane >= o) incl += t;
                 }
                 const uint32_t n_cand = __shfl_sync(0xffffffffu, incl, 31);
-                s_first[wib][lane] = incl - cnt;
-                s_cell[wib][lane] = b;
-                s_pos[wib][lane] = p;
+                s_first[wib][lane] = incl - mine;
                 __syncwarp();
-                uint32_t chunk = 0;  // hits of this chunk so far
+                uint32_t chunk = 0;  // hits of this round so far
                 for (uint32_t r0 = 0; r0 < n_cand; r0 += 32) {
-                    const uint32_t t = r0 + lane;
-                    bool ok = false;
-                    uint32_t qs = 0, so = 0;
-                    if (t < n_cand) {
-                        int owner = 0;  // the last lane whose first entry is <= t
+                    // lanes past the last candidate look at it again and drop it
+                    const uint32_t t = min(r0 + lane, n_cand - 1);
+                    int owner = 0;  // the last lane whose first entry is <= t
 #pragma unroll
-                        for (int st = 16; st; st >>= 1)
-                            if (s_first[wib][owner + st] <= t) owner += st;
-                        ok = exact_extend(v, __ldg(cq + s_cell[wib][owner] + (t - s_first[wib][owner])),
-                                          s_pos[wib][owner], qs, so);
-                    }
+                    for (int st = 16; st; st >>= 1) owner += s_first[wib][owner + st] <= t ? st : 0;
+                    const uint32_t e = t - s_first[wib][owner];
+                    int u = 0;  // its first position whose entries end past e
+#pragma unroll
+                    for (int x = 0; x + 1 < SCAN_POS; ++x) u += s_end[wib][owner][x] <= e;
+                    const uint32_t before = u ? s_end[wib][owner][u - 1] : 0u;
+                    uint32_t qs, so;
+                    const bool ok = exact_extend(v, r0 + lane < n_cand, __ldg(cq + s_cell[wib][owner][u] + (e - before)),
+                                                 (r * SCAN_ROUND + (uint32_t)owner * SCAN_POS + u) * step, qs, so);
+                    __syncwarp();
                     const unsigned m = __ballot_sync(0xffffffffu, ok);
                     const uint32_t nm = (uint32_t)__popc(m);
                     if (MODE == SCAN_STAGE && fits && cursor + total + chunk + nm > stage_cap) {
                         fits = false;
                         if (lane == 0) atomicExch(stage_over, 1u);
                     }
-                    if (WRITE && fits && ok) {
+                    if (fits && ok) {
                         const uint64_t o = out + total + chunk + (uint32_t)__popc(m & ((1u << lane) - 1u));
                         hits[o] = SeedHit{qs, so};
                         if (MODE == SCAN_WRITE) hit_pair[o] = (uint32_t)pair;
@@ -221,29 +255,47 @@ __global__ void __launch_bounds__(256) k_scan(DevLib L, DevQueries Q, int32_t ws
                 total += chunk;
             }
         }
-        if (MODE != SCAN_WRITE && lane == 0) counts[w] = total;
         if (MODE == SCAN_STAGE) {
-            if (lane == 0) stage_start[w] = stage0 + cursor;
+            if (lane == 0) {
+                counts[w] = total;
+                stage_start[w] = stage0 + cursor;
+            }
             cursor += total;
         }
     }
 }
 
-// The staged hits of each pair into pair order: hits[offs[w] ..] = stage[stage_start[w] ..], with
-// the pair id; one warp per pair.
-__global__ void __launch_bounds__(256) k_scan_gather(uint64_t pair0, uint64_t n_pairs, const uint32_t* counts,
-                                                      const uint64_t* offs, const uint32_t* stage_start,
-                                                      const SeedHit* __restrict__ stage, SeedHit* __restrict__ hits,
-                                                      uint32_t* __restrict__ hit_pair) {
+// The hits of the pairs from pair0 on and, from their units' offsets, their own (with one more offset
+// at the end).
+__global__ void __launch_bounds__(256) k_pair_offsets(ScanUnits U, uint32_t n_subjects, uint64_t pair0, uint64_t n_pairs,
+                                                      const uint64_t* __restrict__ unit_offs,
+                                                      uint32_t* __restrict__ counts, uint64_t* __restrict__ offs) {
+    const uint64_t unit0 = scan_unit_of(U, n_subjects, pair0);
+    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p <= n_pairs; p += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t o = unit_offs[scan_unit_of(U, n_subjects, pair0 + p) - unit0];
+        offs[p] = o;
+        if (p < n_pairs)
+            counts[pair0 + p] = (uint32_t)(unit_offs[scan_unit_of(U, n_subjects, pair0 + p + 1) - unit0] - o);
+    }
+}
+
+// The staged hits of each unit into pair order: hits[offs[w] ..] = stage[stage_start[unit0 + w] ..], with
+// the pair id; one warp per unit.
+__global__ void __launch_bounds__(256) k_scan_gather(ScanUnits U, uint32_t n_subjects, uint64_t unit0, uint64_t n_units,
+                                                      const uint32_t* counts, const uint64_t* offs,
+                                                      const uint32_t* stage_start, const SeedHit* __restrict__ stage,
+                                                      SeedHit* __restrict__ hits, uint32_t* __restrict__ hit_pair) {
     const int lane = threadIdx.x & 31;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_pairs; w += nwarps) {
-        const uint32_t c = counts[pair0 + w];
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_units; w += nwarps) {
+        const uint32_t c = counts[unit0 + w];
+        if (!c) continue;
+        const uint32_t pair = (uint32_t)scan_unit(U, n_subjects, unit0 + w).pair;
         const uint64_t o = offs[w];
-        const SeedHit* src = stage + stage_start[pair0 + w];
+        const SeedHit* src = stage + stage_start[unit0 + w];
         for (uint32_t i = lane; i < c; i += 32) {
             hits[o + i] = src[i];
-            hit_pair[o + i] = (uint32_t)(pair0 + w);
+            hit_pair[o + i] = pair;
         }
     }
 }
@@ -2459,43 +2511,62 @@ cudaError_t launch_gather_ops(uint32_t n, const uint32_t* ops, uint32_t ops_cap,
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan(bool write, const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t pair0, uint64_t n_pairs,
-                        uint32_t* counts, const uint64_t* offs, SeedHit* hits, uint32_t* hit_pair, int sms,
-                        cudaStream_t st) {
+cudaError_t launch_scan(const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t pair0, uint64_t n_pairs,
+                        const uint64_t* offs, SeedHit* hits, uint32_t* hit_pair, int sms, cudaStream_t st) {
     const int block = 256;
     const int grid = grid_for(n_pairs * 32, block, 8, sms);
-    if (write)
-        k_scan<SCAN_WRITE><<<grid, block, 0, st>>>(L, Q, ws, pair0, n_pairs, counts, offs, hits, hit_pair, nullptr,
-                                                   0, nullptr, nullptr);
-    else
-        k_scan<SCAN_COUNT><<<grid, block, 0, st>>>(L, Q, ws, pair0, n_pairs, counts, offs, hits, hit_pair, nullptr,
-                                                   0, nullptr, nullptr);
+    k_scan<SCAN_WRITE><<<grid, block, 0, st>>>(L, Q, ws, pair0, n_pairs, ScanUnits{}, nullptr, offs, hits, hit_pair,
+                                               nullptr, 0, nullptr, nullptr);
     return cudaGetLastError();
 }
 
-uint64_t scan_stage_entries(uint64_t n_pairs, int sms) {
-    return (uint64_t)grid_for(n_pairs * 32, 256, 8, sms) * (256 / 32) * SCAN_STAGE_PER_WARP;
+std::vector<uint32_t> scan_segments(uint32_t n_queries, const std::vector<uint32_t>& slen, uint32_t step,
+                                    double hits_per_position, int sms) {
+    // A pair is one warp's while the pairs fill the chip's warp slots twice.  With fewer, a stretch is as
+    // many rounds of the subject as spread the rounds over the slots, and no more than stage a quarter of
+    // SCAN_STAGE_PER_WARP (100 kb at word 7 against 50 consensi: a warp a pair took 5.5 ms, stretches
+    // 0.3; 2.1 Mb, 1.5 M hits in a pair: 50 ms with the pairs' stages overrun, 29 with 14 stretches each).
+    const uint64_t slots = (uint64_t)sms * 128, pairs = (uint64_t)n_queries * slen.size();
+    if (!pairs || pairs >= slots) return {};
+    uint64_t rounds = 0;
+    auto rounds_of = [&](uint32_t n) { return std::max<uint64_t>(1, (n / step + SCAN_ROUND - 1) / SCAN_ROUND); };
+    for (uint32_t n : slen) rounds += rounds_of(n);
+    uint64_t per = (rounds * n_queries + slots - 1) / slots;
+    const double fit = SCAN_STAGE_PER_WARP / 4 / (hits_per_position * SCAN_ROUND + 1.0);
+    if (fit < (double)per) per = (uint64_t)fit;
+    if (per < 1) per = 1;
+    std::vector<uint32_t> first(slen.size() + 1, 0);
+    for (size_t i = 0; i < slen.size(); ++i) first[i + 1] = first[i] + (uint32_t)((rounds_of(slen[i]) + per - 1) / per);
+    return first;
 }
 
-cudaError_t launch_scan_stage(const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t n_pairs, uint32_t* counts,
-                              uint32_t* stage_start, SeedHit* stage, unsigned int* stage_over, int sms,
+uint64_t scan_stage_entries(uint64_t n_units, int sms) {
+    return (uint64_t)grid_for(n_units * 32, 256, 8, sms) * (256 / 32) * SCAN_STAGE_PER_WARP;
+}
+
+cudaError_t launch_scan_stage(const DevLib& L, const DevQueries& Q, int32_t ws, const ScanUnits& U, uint64_t n_units,
+                              uint32_t* counts, uint32_t* stage_start, SeedHit* stage, unsigned int* stage_over, int sms,
                               cudaStream_t st, bool queue) {
-    // stage_over: [0] the overflow flag, [2..3] the pair queue (both zeroed by the caller); without
-    // `queue` the warps take pairs by stride
+    // stage_over: [0] the overflow flag, [2..3] the unit queue (both zeroed by the caller); without
+    // `queue` the warps take units by stride
     const int block = 256;
-    const int grid = grid_for(n_pairs * 32, block, 8, sms);
-    k_scan<SCAN_STAGE><<<grid, block, 0, st>>>(L, Q, ws, 0, n_pairs, counts, nullptr, stage, nullptr, stage_start,
+    const int grid = grid_for(n_units * 32, block, 8, sms);
+    k_scan<SCAN_STAGE><<<grid, block, 0, st>>>(L, Q, ws, 0, n_units, U, counts, nullptr, stage, nullptr, stage_start,
                                                SCAN_STAGE_PER_WARP, stage_over,
                                                queue ? reinterpret_cast<unsigned long long*>(stage_over + 2) : nullptr);
     return cudaGetLastError();
 }
-
-cudaError_t launch_scan_gather(uint64_t pair0, uint64_t n_pairs, const uint32_t* counts, const uint64_t* offs,
-                               const uint32_t* stage_start, const SeedHit* stage, SeedHit* hits, uint32_t* hit_pair,
-                               int sms, cudaStream_t st) {
-    if (!n_pairs) return cudaSuccess;
-    k_scan_gather<<<grid_for(n_pairs * 32, 256, 8, sms), 256, 0, st>>>(pair0, n_pairs, counts, offs, stage_start,
-                                                                       stage, hits, hit_pair);
+cudaError_t launch_scan_gather(const ScanUnits& U, uint32_t n_subjects, uint64_t unit0, uint64_t n_units,
+                               const uint32_t* counts, const uint64_t* offs, const uint32_t* stage_start,
+                               const SeedHit* stage, SeedHit* hits, uint32_t* hit_pair, int sms, cudaStream_t st) {
+    if (!n_units) return cudaSuccess;
+    k_scan_gather<<<grid_for(n_units * 32, 256, 8, sms), 256, 0, st>>>(U, n_subjects, unit0, n_units, counts, offs,
+                                                                       stage_start, stage, hits, hit_pair);
+    return cudaGetLastError();
+}
+cudaError_t launch_pair_offsets(const ScanUnits& U, uint32_t n_subjects, uint64_t pair0, uint64_t n_pairs,
+                                const uint64_t* unit_offs, uint32_t* counts, uint64_t* offs, int sms, cudaStream_t st) {
+    k_pair_offsets<<<grid_for(n_pairs + 1, 256, 8, sms), 256, 0, st>>>(U, n_subjects, pair0, n_pairs, unit_offs, counts, offs);
     return cudaGetLastError();
 }
 

@@ -3,25 +3,41 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "rmb_device.cuh"
 
 namespace rmb {
 
-cudaError_t launch_scan(bool write, const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t pair0, uint64_t n_pairs,
-                        uint32_t* counts, const uint64_t* offs, SeedHit* hits, uint32_t* hit_pair, int sms,
-                        cudaStream_t st);
-// Single-pass scan: counts plus the hits staged per warp (scan_stage_entries(n_pairs, sms)
-// SeedHits of stage), then k_scan_gather puts a range of pairs' hits in pair order at their offsets.  A set
-// *stage_over (a warp's stretch of SCAN_STAGE_PER_WARP entries ran out) means the staged hits are
-// incomplete: the caller runs launch_scan(write) instead.
+// Every pair's hits in place, at the pairs' offsets.
+cudaError_t launch_scan(const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t pair0, uint64_t n_pairs,
+                        const uint64_t* offs, SeedHit* hits, uint32_t* hit_pair, int sms, cudaStream_t st);
+// Scan units: the (query, subject) pairs, or, with per_query > 0, stretches of them: first[s] .. first[s + 1]
+// of a query's per_query units are subject s's, subject[u] is unit u's.
+struct ScanUnits {
+    const uint32_t* first = nullptr;
+    const uint32_t* subject = nullptr;
+    uint32_t per_query = 0;
+};
+// `first` for stretches that suit the launch (empty: whole pairs); step is the scan stride in bases,
+// hits_per_position the expected word hits of a scan position of the longest query.
+std::vector<uint32_t> scan_segments(uint32_t n_queries, const std::vector<uint32_t>& slen, uint32_t step,
+                                    double hits_per_position, int sms);
+// Single-pass scan: counts per unit plus the hits staged per warp (scan_stage_entries(n_units, sms)
+// SeedHits of stage), then k_scan_gather puts a range of units' hits in pair order at the units' offsets.
+// A set *stage_over (a warp's stretch of SCAN_STAGE_PER_WARP entries ran out) means the staged hits are
+// incomplete: the caller runs launch_scan instead.  launch_pair_offsets: pairs' counts and offsets from
+// their units' offsets.
 constexpr uint32_t SCAN_STAGE_PER_WARP = 32768;
-uint64_t scan_stage_entries(uint64_t n_pairs, int sms);
-cudaError_t launch_scan_stage(const DevLib& L, const DevQueries& Q, int32_t ws, uint64_t n_pairs, uint32_t* counts,
-                              uint32_t* stage_start, SeedHit* stage, unsigned int* stage_over, int sms,
+uint64_t scan_stage_entries(uint64_t n_units, int sms);
+cudaError_t launch_scan_stage(const DevLib& L, const DevQueries& Q, int32_t ws, const ScanUnits& U, uint64_t n_units,
+                              uint32_t* counts, uint32_t* stage_start, SeedHit* stage, unsigned int* stage_over, int sms,
                               cudaStream_t st, bool queue);
-cudaError_t launch_scan_gather(uint64_t pair0, uint64_t n_pairs, const uint32_t* counts, const uint64_t* offs,
-                               const uint32_t* stage_start, const SeedHit* stage, SeedHit* hits, uint32_t* hit_pair,
-                               int sms, cudaStream_t st);
+cudaError_t launch_scan_gather(const ScanUnits& U, uint32_t n_subjects, uint64_t unit0, uint64_t n_units,
+                               const uint32_t* counts, const uint64_t* offs, const uint32_t* stage_start,
+                               const SeedHit* stage, SeedHit* hits, uint32_t* hit_pair, int sms, cudaStream_t st);
+cudaError_t launch_pair_offsets(const ScanUnits& U, uint32_t n_subjects, uint64_t pair0, uint64_t n_pairs,
+                                const uint64_t* unit_offs, uint32_t* counts, uint64_t* offs, int sms, cudaStream_t st);
 // queue: 8 bytes of device scratch (the hit queue counter; zeroed here)
 cudaError_t launch_ungapped(const DevLib& L, const DevQueries& Q, const DevParams* P, int32_t ucut, uint64_t n,
                             const SeedHit* hits, const uint32_t* hit_pair, UngBox* out, int sms, cudaStream_t st,
