@@ -2797,12 +2797,7 @@ static cudaError_t pack_launch(const DevParams* P, uint64_t n, const PrelimGeo* 
         K.q_nib = dp_nibbles(cfg.q_dp, 4, cfg.q_stride);
         K.s_nib = dp_nibbles(cfg.s_dp, 2, cfg.s_stride);
         K.neg_go = pack2(-cfg.gap_open, -cfg.gap_open);
-        for (int c = 0; c < DUAL_W; ++c) {
-            K.neg_ge[c] = pack2(-cfg.gap_extend * c, -cfg.gap_extend * c);
-            K.pos_ge[c] = pack2(cfg.gap_extend * c, cfg.gap_extend * c);
-        }
         K.one = 1;
-        K.minus_one = 0xffffffffu;
         const uint64_t want = (n + 2 * DUAL_BLOCK - 1) / (2 * DUAL_BLOCK), cap = (uint64_t)sms * dual_sm;
         if (plain)
             k_prelim_dual<false><<<(unsigned)want, DUAL_BLOCK, 0, st>>>(P, K, n, geo, out, cfg.list, cfg.list_ctl, n_wide + 1,

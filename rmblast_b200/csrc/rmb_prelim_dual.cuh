@@ -11,26 +11,42 @@
 // depend on each other through the gap and the running best only, one operation each, so the
 // arithmetic pipe stays busy on the other ten.
 //
-// Bound: the half-rate integer pipe (packed add-max, byte permutes, compares) and, behind it, issue.
+// Bound: the half-rate integer pipe (packed add-max, byte permutes, compares; 74 % of its rate) and the
+// latency of a row's chain with 12 warps an SM, what the rows in registers leave.
 // A live test is one half-precision compare: the values are below 0x7c00 and not negative, so their
 // order as half floats is their order as integers; the cell is then kept or cleared by a half-precision
 // product with 1 or 0, and the live columns are counted into bit masks by half-precision
-// multiply-adds (1024 + sums of 2^c, exact), both on the otherwise idle multiply-add pipe.
+// multiply-adds (1024 + sums of 2^c, exact), both on the otherwise idle multiply-add pipe.  The
+// threshold (running best - X) moves from column to column in its own coordinate: one add-max, and
+// one multiply-add for the diagonal's gap_extend, no constant a column.
 //
-// Measured (B200): 755 G cells/s on 1.07 M records, 0.8 warp instructions a cell, against 380 G and
-// 2.4 for k_prelim_stream (a cell step a thread, the band in shared memory); the preliminary DP of
-// 120 queries of 60 kb went 95 -> 55 ms, of 1,000 contigs 414 -> 243 ms, k_prelim_pack included.  A
-// window of 56 diagonals lets 0.6 % of random word hits outgrow it (48: 5 %), and H and E of two
-// records fill the register file at 8 warps an SM.
+// Columns that are dead in all of a warp's 64 records are left out, four at a time: on the left where no
+// cell of the last row lives there or in the column behind (the vertical gap's), on the right where
+// no cell lives and no horizontal gap reaches in.  Of the 56 columns 16 % go so on random word hits;
+// the inner ones are never dead in all 64.
 //
-// Rows run in batches of DUAL_ROWS; records end, start and move their windows between batches.  A
-// record that ends inside a batch runs on for the rest of it: past the subject's end the rows score
-// as blocked, past the query's the columns do, so no best changes, and its cells are not counted.
+// A record starts in a half without clearing it: its origin is set so high that what the half's last
+// record left, at most its best, stays below best - X and dies at the first look; the first row's
+// cells are written over it.  So the values climb from record to record, until DUAL_REBASE.
+//
+// Measured (B200), preliminary DP with k_prelim_pack's part: 120 queries of 60 kb 95 ms with
+// k_prelim_stream (a cell step a thread, the band in shared memory), 55 with this kernel in batches
+// of 4 rows, cleared at every start, 8 warps an SM and a constant a column, 44 as it is; 1,000
+// contigs 414, 243 and 191 ms; 1,060 G cells/s at 0.63 warp instructions a cell (k_prelim_stream: 380 G
+// at 2.4).  A window of 56 diagonals lets 0.6 % of random word hits outgrow it (48: 5 %).
+//
+// Rows run in batches of DUAL_ROWS (bulk of 1,000 contigs: 4 rows 227 ms, 6 213, 8 208, before the
+// last of the above); records end, start and move their windows between batches.  A record that
+// ends inside a batch runs on for the rest of it: past the subject's end the rows score as blocked,
+// past the query's the columns do, so no best changes, and its cells are not counted.
 #include "rmb_prelim_pack.cuh"
 
 namespace rmb {
 
-constexpr int DUAL_W = 56, DUAL_K = 26, DUAL_ROWS = 4, DUAL_SHIFT = 4, DUAL_BLOCK = 128;
+constexpr int DUAL_W = 56, DUAL_K = 26, DUAL_ROWS = 8, DUAL_SHIFT = 4, DUAL_BLOCK = 128;
+// best + origin may pass DUAL_REBASE by a batch, a window move and a record's start (under 1,100) and a
+// cell lies 63 * 55 above at most: below 0x7c00; what is left after the move keeps live values above 255
+constexpr int32_t DUAL_REBASE = 24576, DUAL_REBASE_BY = 24064;
 constexpr int DUAL_BITS = 10;  // columns of a half-precision bit mask
 constexpr int DUAL_MASKS = (DUAL_W + DUAL_BITS - 1) / DUAL_BITS;
 
@@ -39,9 +55,7 @@ struct DualConst {
     const uint8_t *q_dp, *s_dp;   // the byte copies that the records point into
     const uint32_t *q_nib, *s_nib;  // their codes, eight to a word
     uint32_t neg_go;
-    uint32_t neg_ge[DUAL_W];      // -gap_extend * c
-    uint32_t pos_ge[DUAL_W];      // gap_extend * c
-    uint32_t one, minus_one;      // 1 and -1: factors the compiler does not see keep an add on the multiply-add pipe
+    uint32_t one;  // 1: a factor the compiler does not see keeps an add on the multiply-add pipe
 };
 
 __device__ __forceinline__ uint32_t half_ge(uint32_t a, uint32_t b) {  // 1.0 or 0.0 per half
@@ -75,7 +89,7 @@ struct DualCold {
 };
 
 template <bool QUEUE>
-__global__ void __launch_bounds__(DUAL_BLOCK)
+__global__ void __launch_bounds__(DUAL_BLOCK, 3)
 k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst K, uint64_t n_rec,
               const PrelimGeo* __restrict__ geo, PrelimOut* __restrict__ out, uint32_t* __restrict__ list,
               unsigned int* __restrict__ n_list, unsigned int* __restrict__ queue,
@@ -104,13 +118,13 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
         order_end = dc.order_end;
     }
     const StreamDiv div_ge(ge);
-    const uint32_t step2 = pack2(2 * ge, 2 * ge);
+    const uint32_t step2 = pack2(2 * ge, 2 * ge), ge2 = pack2(ge, ge);
 
     uint32_t H[W], E[W], s[2][7];
 #pragma unroll
     for (int c = 0; c < W; ++c) H[c] = E[c] = 0;
     int phase[2] = {0, 0};  // 0 needs a record, 1 left extension, 2 right extension, 4 no records left
-    uint32_t pb = pack2(PACK_REBASE_BY, PACK_REBASE_BY), xp = 0;  // best + origin; X
+    uint32_t pb = pack2(DUAL_REBASE - DUAL_REBASE_BY, DUAL_REBASE - DUAL_REBASE_BY), xp = 0, nx = 0;  // nx: -X  // best + origin; X
     int32_t org[2] = {0, 0}, rows[2] = {0, 0}, kr[2] = {0, 0};    // rows: rows left; kr as k_prelim_pack's
     uint32_t rec[2] = {0, 0};
     uint32_t ended = 3, failed = 0;  // bit h: half h's extension is over; it goes to the list
@@ -120,7 +134,13 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
         if (QUEUE) return atomicAdd(queue, 1u);
         return taken < 2 ? (blockIdx.x * DUAL_BLOCK + threadIdx.x) * 2 + taken++ : 0xffffffffu;
     };
-    uint32_t next_t = take();
+    uint32_t next_t = take(), next_id = 0;
+    bool known = false;  // next_id is next_t's record
+    auto resolve = [&]() -> uint32_t {
+        return !order ? next_t : next_t < n_front ? order[next_t] : order[order_end - 1 - (uint64_t)(next_t - n_front)];
+    };
+    uint32_t fetched = 0xffffffffu;
+    uint32_t un = 0;  // live outer columns of the warp's last row: bit c of the first 13, bit c - 24 of those from 40 on
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -128,11 +148,13 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
 
     for (;;) {
         if (__any_sync(FULL, (ended & 1u && phase[0] != 4) || (ended & 2u && phase[1] != 4))) {
-            uint32_t keep = FULL, vj = 0;  // halves that run on; the new ones' J
+            uint32_t vj = 0;  // the new halves' J
             int32_t base[2] = {0, 0};
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 DualCold& k = cold[h][threadIdx.x];
+                // a first step adds 127 at most to what the half still holds, all of it at most its best
+                const int32_t top = (int32_t)(h ? pb >> 16 : pb & 0xffffu) + 128;
                 while ((ended >> h & 1u) && phase[h] != 4) {
                     const int32_t best = (int32_t)((h ? pb >> 16 : pb & 0xffffu)) - org[h];
                     if (phase[h] != 0) {
@@ -155,16 +177,17 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                         }
                     }
                     failed &= ~(1u << h);
-                    keep &= h ? 0x0000ffffu : 0xffff0000u;
                     if (phase[h] == 0) {
                         if (next_t >= n_rec) {
                             phase[h] = 4;
-                            pb = h ? (pb & 0xffffu) | (uint32_t)PACK_REBASE_BY << 16 : (pb & 0xffff0000u) | PACK_REBASE_BY;
+                            pb = h ? (pb & 0xffffu) | (uint32_t)top << 16 : (pb & 0xffff0000u) | (uint32_t)top;
                             xp &= h ? 0x0000ffffu : 0xffff0000u;
+                            nx &= h ? 0x0000ffffu : 0xffff0000u;
                             break;
                         }
-                        k.t = !order ? next_t : next_t < n_front ? order[next_t] : order[order_end - 1 - (uint64_t)(next_t - n_front)];
+                        k.t = known ? next_id : resolve();
                         next_t = take();
+                        known = false;
                         rec[h] = 0;
                         k.l_score = 0;
                         phase[h] = 1;
@@ -184,7 +207,7 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                         m = (int32_t)g1.y - m;
                         nb = (int32_t)g1.x - nb;
                     }
-                    org[h] = X + 256;
+                    org[h] = top + X;
                     pb = h ? (pb & 0xffffu) | (uint32_t)org[h] << 16 : (pb & 0xffff0000u) | (uint32_t)org[h];
                     if (m <= 0 || nb <= 0) continue;  // an empty extension: score 0
                     const int32_t jmax = (int32_t)div_ge((uint32_t)(X - goe)) + 1;
@@ -211,6 +234,7 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                     rec[h] += (uint32_t)J + 1;
                     base[h] = org[h] + ge * DUAL_K;
                     xp = h ? (xp & 0xffffu) | (uint32_t)X << 16 : (xp & 0xffff0000u) | (uint32_t)X;
+                    nx = h ? (nx & 0xffffu) | (uint32_t)(-X) << 16 : (nx & 0xffff0000u) | ((uint32_t)(-X) & 0xffffu);
                     vj |= (uint32_t)J << (16 * h);
                     ended &= ~(1u << h);
                 }
@@ -220,26 +244,20 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
             // the initial rows (gapped.rs:165-200): cell 0, gap cells 1 .. J; cell J's diagonal leads out
             // of the first row's band
             const uint32_t fresh = prmt((vj + 0x7fff7fffu), 0, 0xbb99);  // halves with a new J (J >= 1)
-#pragma unroll
-            for (int c = 0; c < W; ++c) {
-                H[c] &= keep;
-                E[c] &= keep;
-            }
             const uint32_t v1 = pack2(base[0] - go, base[1] - go), v2 = pack2(base[0] - 2 * go, base[1] - 2 * go);
-            H[DUAL_K] |= pack2(base[0], base[1]) & fresh;
-            E[DUAL_K] |= v1 & fresh;
+            H[DUAL_K] = (H[DUAL_K] & ~fresh) | (pack2(base[0], base[1]) & fresh);
+            E[DUAL_K] = (E[DUAL_K] & ~fresh) | (v1 & fresh);
             uint32_t in = fresh;  // halves with gap cell i
 #pragma unroll
             for (int i = 1; i <= 16; ++i) {
                 const uint32_t in1 = prmt(vj + 0x80008000u - (uint32_t)(i + 1) * 0x00010001u, 0, 0xbb99);
-                E[DUAL_K + i] |= v2 & in;
-                H[DUAL_K + i] |= v1 & in1;
+                E[DUAL_K + i] = (E[DUAL_K + i] & ~in) | (v2 & in);
+                H[DUAL_K + i] = (H[DUAL_K + i] & ~in1) | (v1 & in1);
                 in = in1;
             }
+            un |= 0x7u << 16;  // cells 14 .. 16 of the initial rows
         }
 
-        if (next_t < n_rec && !order)  // the next record's geometry, for when one of the two ends
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(geo + next_t));
         // ---- the residues of a batch of rows
         uint32_t pend[2], aw[2];
 #pragma unroll
@@ -265,11 +283,20 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
             const uint2 ta = tab[aw[0] & 15u], tb = tab[aw[1] & 15u];
             aw[0] >>= 4;
             aw[1] >>= 4;
-            uint32_t p = pb, f = 0, al[DUAL_MASKS];
+            uint32_t w = pb - xp, f = 0, al[DUAL_MASKS];  // w: the running best - X, at the next column's diagonal
+            int end = W;
 #pragma unroll
             for (int i = 0; i < DUAL_MASKS; ++i) al[i] = 0x64006400u;
 #pragma unroll
             for (int g = 0; g < W / 4; ++g) {
+                if (g < 3 && !(un & ((1u << (4 * g + 5)) - 1u))) {
+                    w += 4 * ge2;
+                    continue;
+                }
+                if (g >= 10 && !(un >> (4 * g - 24)) && !__any_sync(FULL, half_ge(f, w) != 0)) {
+                    end = 4 * g;
+                    break;
+                }
                 const uint32_t ga = prmt(ta.x, ta.y, g & 1 ? s[0][g / 2] >> 16 : s[0][g / 2]);
                 const uint32_t gb = prmt(tb.x, tb.y, g & 1 ? s[1][g / 2] >> 16 : s[1][g / 2]);
 #pragma unroll
@@ -280,15 +307,16 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                     const uint32_t t = __viaddmax_s16x2(H[c], sc, up);
                     const uint32_t cell = __vmaxs2(t, f);
                     f = __viaddmax_s16x2(t, K.neg_go, f);
-                    p = __viaddmax_s16x2(t, K.neg_ge[c], p);
-                    const uint32_t thr = xp * K.minus_one + (p * K.one + K.pos_ge[c]);
+                    const uint32_t thr = __viaddmax_s16x2(t, nx, w);
+                    w = thr * K.one + ge2;
                     const uint32_t live = half_ge(cell, thr);
                     H[c] = half_mul(cell, live);
                     al[c / DUAL_BITS] = half_fma(live, (uint32_t)(0x3c00 + 0x400 * (c % DUAL_BITS)) * 0x00010001u, al[c / DUAL_BITS]);
                     E[c] = __viaddmax_s16x2(H[c], K.neg_go, up);
                 }
             }
-            pb = p;
+            pb = w + xp - ge2 * (uint32_t)end;
+            un = 0;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -299,6 +327,7 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
 #pragma unroll
                 for (int i = 0; i < DUAL_MASKS; ++i) m[i] = (h ? al[i] >> 16 : al[i]) & 0x3ffu;
                 const uint32_t lo = m[0] | m[1] << 10 | m[2] << 20, hi = m[3] | m[4] << 10 | m[5] << 20;
+                un |= (lo & 0x1fffu) | hi >> 10 << 16;
                 fc[h] = lo ? __ffs((int)lo) - 1 : 29 + __ffs((int)hi);
                 lc[h] = hi ? 61 - __clz((int)hi) : 31 - __clz((int)lo);
                 --rows[h];
@@ -321,6 +350,16 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                     }
                 }
             }
+            un = __reduce_or_sync(FULL, un);
+        }
+
+        // the next record, found while rows run: its number, then its geometry's line
+        if (known) {
+            if (next_id != fetched && next_t < n_rec) asm volatile("prefetch.global.L1 [%0];" ::"l"(geo + next_id));
+            fetched = next_id;
+        } else if (next_t < n_rec) {
+            next_id = resolve();
+            known = true;
         }
 
         // ---- between the batches: records that reached the cutoff, window moves, origins
@@ -329,20 +368,21 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
         for (int h = 0; h < 2; ++h) {
             org[h] += 2 * ge * DUAL_ROWS;
             const int32_t bo = (int32_t)(h ? pb >> 16 : pb & 0xffffu);
-            if (bo > PACK_REBASE) down |= 1u << h;
+            if (bo > DUAL_REBASE) down |= 1u << h;
             if (!(ended >> h & 1u)) {
                 if (bo - org[h] + (phase[h] == 2 ? cold[h][threadIdx.x].l_score : 0) >= cutoff) {
                     ended |= 1u << h;
                     failed |= 1u << h;
-                } else if (lc[h] > W - 8 && fc[h] > DUAL_SHIFT + 6) {
+                } else if (lc[h] > W - 12 && fc[h] > DUAL_SHIFT + 8) {
                     right |= 1u << h;
-                } else if (fc[h] < 6 && lc[h] < W - DUAL_SHIFT - 8) {
+                } else if (fc[h] < 9 && lc[h] < W - DUAL_SHIFT - 10) {
                     left |= 1u << h;
                 }
             }
         }
         if (__any_sync(FULL, right | left | down)) {
             if (__any_sync(FULL, right)) {
+                un |= (un & 0x1fffu) >> DUAL_SHIFT | 0x1fffu >> (13 - DUAL_SHIFT) << (13 - DUAL_SHIFT);
                 const uint32_t sel = (right & 1u ? 0x54u : 0x10u) | (right & 2u ? 0x7600u : 0x3200u);
 #pragma unroll
                 for (int c = 0; c < W; ++c) {
@@ -351,6 +391,7 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                 }
             }
             if (__any_sync(FULL, left)) {
+                un |= ((un >> 16 << DUAL_SHIFT) | ((1u << DUAL_SHIFT) - 1u)) << 16;
                 const uint32_t sel = (left & 1u ? 0x54u : 0x10u) | (left & 2u ? 0x7600u : 0x3200u);
 #pragma unroll
                 for (int c = W - 1; c >= 0; --c) {
@@ -389,9 +430,9 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
                     }
                 }
                 if (down >> h & 1u) {
-                    by |= (uint32_t)(0x10000 - PACK_REBASE_BY) << (16 * h);
-                    org[h] -= PACK_REBASE_BY;
-                    pb -= (uint32_t)PACK_REBASE_BY << (16 * h);
+                    by |= (uint32_t)(0x10000 - DUAL_REBASE_BY) << (16 * h);
+                    org[h] -= DUAL_REBASE_BY;
+                    pb -= (uint32_t)DUAL_REBASE_BY << (16 * h);
                 }
             }
             if (__any_sync(FULL, down)) {

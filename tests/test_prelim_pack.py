@@ -60,3 +60,25 @@ def test_packed_rows_match_the_warp_kernel(gaps, pipeline):
     assert len(got[0][0]) > 100
     assert np.array_equal(got[0][0], got[1][0])
     assert got[0][1:] == got[1][1:]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gaps", [(20, 5, 100, 150), (20, 55, 128, 150)])
+def test_many_records_a_thread(gaps):
+    """Millions of random word hits: each half of a k_prelim_dual thread runs tens of records one after the
+    other (their values climb until they are moved down), also at nearly the steepest gap it takes."""
+    rng = np.random.default_rng([0x9ACD, *gaps[:3]])
+    lib = [synth.random_dna(rng, int(k)) for k in rng.integers(60, 6000, 60)]
+    qs = [synth.plant(rng, synth.random_dna(rng, n), lib, 0.05, None, (0.05, 0.3), (0.01, 0.05)) for n in (250_000, 60_000)]
+    db = api.SubjectDb.from_records([(f"s{i}", s) for i, s in enumerate(lib)])
+    m = api.ScoreMatrix.from_text(synth.MATRIX_TEXT, synth.MATRIX_NAME)
+    enc = [api.encode(q) for q in qs]
+    got = []
+    for kernels in (0, 1):
+        s = api.Searcher(api.SearchParams(gap_open=gaps[0], gap_extend=gaps[1], word_size=7, xdrop_ungap=400,
+                                          xdrop_gap=gaps[2], xdrop_gap_final=200, min_raw_gapped_score=gaps[3],
+                                          complexity_adjust=True, kernels=kernels), m, db)
+        res = s.search(enc)
+        got.append((res.counters["so_cells"], res.counters["prelims"], res.counters["ungapped"], res.tabular(FIELDS)))
+    assert got[0][2] > 10 * 148 * 3 * 128 * 2  # halves of 12 warps on each of 148 SMs
+    assert got[0] == got[1]
