@@ -362,7 +362,7 @@ void mask_queries(rmb_ctx& C, rmb_queries& QH, bool compat, rmb_counters& ctr) {
     EvTimer ev;
     ev.start(st);
     dust_queries(C, QH, QH.d_qm.as<uint8_t>(), compat, nullptr, nullptr, st, ctr);
-    CK(launch_revcomp(QH.d_qm.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq,
+    CK(launch_revcomp(QH.d_qm.as<uint8_t>(), QH.d_off.as<uint64_t>(), QH.d_len.as<uint32_t>(), nq, QH.host.size(),
                       QH.d_qmrc.as<uint8_t>(), st));
     ev.stop(st);
     ctr.launches += 1;
@@ -1829,7 +1829,7 @@ static rmb_queries* make_queries(rmb_ctx* C, uint32_t nq, const uint8_t* const* 
         CK(cudaMemcpyAsync(H->d_q.p, H->host.data(), tot, cudaMemcpyHostToDevice, st));
         upload(H->d_off, H->off, st);
         upload(H->d_len, H->len, st);
-        CK(launch_revcomp(H->d_q.as<uint8_t>(), H->d_off.as<uint64_t>(), H->d_len.as<uint32_t>(), nq,
+        CK(launch_revcomp(H->d_q.as<uint8_t>(), H->d_off.as<uint64_t>(), H->d_len.as<uint32_t>(), nq, H->host.size(),
                           H->d_qrc.as<uint8_t>(), st));
         CK(cudaStreamSynchronize(st));
         return H;
@@ -2033,7 +2033,7 @@ void run_search(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_
         CH->d_qm.ensure(hm.size());
         CH->d_qmrc.ensure(hm.size());
         CK(cudaMemcpy(CH->d_qm.p, hm.data(), hm.size(), cudaMemcpyHostToDevice));
-        CK(launch_revcomp(CH->d_qm.as<uint8_t>(), CH->d_off.as<uint64_t>(), CH->d_len.as<uint32_t>(), CH->n,
+        CK(launch_revcomp(CH->d_qm.as<uint8_t>(), CH->d_off.as<uint64_t>(), CH->d_len.as<uint32_t>(), CH->n, CH->host.size(),
                           CH->d_qmrc.as<uint8_t>(), C.st));
         CK(cudaStreamSynchronize(C.st));
         ctr.launches += 1;

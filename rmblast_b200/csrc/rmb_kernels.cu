@@ -2479,6 +2479,13 @@ __global__ void k_traceback_join(const DevParams* __restrict__ P, uint32_t n, co
     out[t] = o;
 }
 
+// Blocks a query in the kernels that go over every position of every query: one for 4,096 positions of a
+// query of the mean length.  (One block a query left a 2.1 Mb query to 512 threads: its lookup
+// codes took 4.7 ms, 0.1 now, its reverse complement 4.6; a query of 60 kb 0.32 and 0.1.)
+static unsigned query_parts(uint64_t positions, uint32_t nq) {
+    return (unsigned)std::min<uint64_t>(positions / nq / 4096 + 1, 1024);
+}
+
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
@@ -2857,8 +2864,7 @@ cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t
     if (!nq) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(out, PACK_BLOCKED, 4 * stride, st);
     if (e != cudaSuccess) return e;
-    const uint64_t parts = stride / nq / 4096 + 1;
-    k_dp_query<<<dim3(nq, (unsigned)std::min<uint64_t>(parts, 1024)), 256, 0, st>>>(q, qrc, off, len, out, stride);
+    k_dp_query<<<dim3(nq, query_parts(stride, nq)), 256, 0, st>>>(q, qrc, off, len, out, stride);
     return dp_pack(out, 4, stride, 0, st);
 }
 
@@ -3164,7 +3170,8 @@ __global__ void k_lut_codes(DevQueries Q, int32_t ws, const uint64_t* __restrict
     const uint64_t cbase = Q.cs_off[qi];
     const uint32_t total = 2 * n + 1;
     const bool ok = (int64_t)ws <= (int64_t)n;  // each context is n bases long
-    for (uint32_t s = threadIdx.x; s < total; s += blockDim.x) {
+    for (uint64_t at = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; at < total; at += (uint64_t)gridDim.y * blockDim.x) {
+        const uint32_t s = (uint32_t)at;
         uint32_t code = NO_CODE;
         if (ok && s != n) {
             // context 0 = [0, n-1], context 1 = [n+1, 2n]
@@ -3209,20 +3216,28 @@ __global__ void k_lut_place(uint64_t n_valid, const uint32_t* __restrict__ keys,
 __global__ void k_lut_pv(uint64_t n_words_total, const uint64_t* __restrict__ pv_off, const uint64_t* __restrict__ cs_off,
                          const int32_t* __restrict__ lw, uint32_t nq, const uint32_t* __restrict__ counts,
                          uint32_t* __restrict__ pv) {
-    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words_total;
-         w += (uint64_t)gridDim.x * blockDim.x) {
+    // a warp's 32 words at a time; a word's 32 counts are one load of the warp and one vote
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t w0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; w0 < n_words_total; w0 += nwarps * 32) {
+        const uint64_t w = min(w0 + lane, n_words_total - 1);
         uint32_t lo = 0, hi = nq;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) / 2;
             if (pv_off[mid] <= w) lo = mid;
             else hi = mid;
         }
-        const uint64_t cells = 1ull << (2 * lw[lo]);
-        const uint64_t c0 = (w - pv_off[lo]) * 32;
+        const uint64_t c0 = (w - pv_off[lo]) * 32, cell = cs_off[lo] + c0;
+        const uint32_t n = (uint32_t)min((unsigned long long)32, (1ull << (2 * lw[lo])) - c0);
         uint32_t bits = 0;
-        for (uint32_t b = 0; b < 32 && c0 + b < cells; ++b)
-            if (counts[cs_off[lo] + c0 + b]) bits |= 1u << b;
-        pv[w] = bits;
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const uint64_t at = __shfl_sync(0xffffffffu, cell, k);
+            const bool some = lane < __shfl_sync(0xffffffffu, n, k) && counts[at + lane];
+            const uint32_t word = __ballot_sync(0xffffffffu, some);
+            if (lane == (uint32_t)k) bits = word;
+        }
+        if (w0 + lane < n_words_total) pv[w] = bits;
     }
 }
 
@@ -3243,7 +3258,7 @@ cudaError_t launch_lut_build(const DevQueries& Q, int32_t ws, uint32_t nq, const
     }
     e = cudaMemsetAsync(counts, 0, (n_cells + 1) * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    k_lut_codes<<<nq, 512, 0, st>>>(Q, ws, pos_off, keys, vals, counts);
+    k_lut_codes<<<dim3(nq, query_parts(n_pos, nq)), 512, 0, st>>>(Q, ws, pos_off, keys, vals, counts);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     size_t tb = temp_bytes;
     e = cub::DeviceScan::ExclusiveSum(temp, tb, counts, cs, (int64_t)n_cells + 1, st);
@@ -3270,7 +3285,8 @@ cudaError_t launch_lut_build(const DevQueries& Q, int32_t ws, uint32_t nq, const
 }  // namespace rmb
 
 namespace rmb {
-// reverse complement of every sentinel-wrapped query (encoding.rs:136 revcomp_blastna)
+// reverse complement of every sentinel-wrapped query (encoding.rs:136 revcomp_blastna), a block column a
+// query (see query_parts)
 __global__ void k_revcomp(const uint8_t* __restrict__ q, const uint64_t* __restrict__ off,
                           const uint32_t* __restrict__ len, uint8_t* __restrict__ rc) {
     __shared__ uint8_t comp[16];
@@ -3280,14 +3296,15 @@ __global__ void k_revcomp(const uint8_t* __restrict__ q, const uint64_t* __restr
     }
     __syncthreads();
     const uint64_t o = off[blockIdx.x];
-    const uint32_t n = len[blockIdx.x] + 2;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) rc[o + i] = comp[q[o + n - 1 - i] & 15];
+    const uint64_t n = (uint64_t)len[blockIdx.x] + 2;
+    for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.y * blockDim.x)
+        rc[o + i] = comp[q[o + n - 1 - i] & 15];
 }
 
-cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint8_t* rc,
-                           cudaStream_t st) {
+cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint64_t bytes,
+                           uint8_t* rc, cudaStream_t st) {
     if (!nq) return cudaSuccess;
-    k_revcomp<<<nq, 256, 0, st>>>(q, off, len, rc);
+    k_revcomp<<<dim3(nq, query_parts(bytes, nq)), 256, 0, st>>>(q, off, len, rc);
     return cudaGetLastError();
 }
 

@@ -210,7 +210,7 @@ cudaError_t launch_lut_build(const DevQueries& Q, int32_t ws, uint32_t nq, const
 }  // namespace rmb
 
 namespace rmb {
-cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint8_t* rc,
+cudaError_t launch_revcomp(const uint8_t* q, const uint64_t* off, const uint32_t* len, uint32_t nq, uint64_t bytes, uint8_t* rc,
                            cudaStream_t st);
 // DUST masking of a query batch in segments (k_dust_segments): unit_off[i] is query i's first unit of
 // `seg` starts (dust_segment_starts), rnd the first rnd_cap bases the N draw, conv, n_n, mk (zeroed),
