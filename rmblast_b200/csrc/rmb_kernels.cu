@@ -363,11 +363,9 @@ __device__ __forceinline__ void extend_ungapped(const uint8_t* query, int64_t q_
 // takes the next hit index from the grid-wide queue (one atomic per warp and round), so lanes do
 // not wait for the longest walk of the warp.  Same arithmetic as extend_ungapped + the box of
 // engine.rs:1165-1170 / 1244-1261.
-// 16 steps a round: the walks at the default size run hundreds of bases, so fewer refills pay
-// for the idle steps after a walk ends (8 measured 49-50 ms, 16 47 ms a step).  Four bases a
-// step with their loads issued together measured slower, on this kernel (27 -> 32 ms a step on
-// 1,000 queries of 1-200 kb) and in the fused dedup's lane walks
-constexpr int UNG_GROUP = 16;
+// UNG_GROUP steps of eight bases a round: the walks at the default size run hundreds of bases, so
+// fewer refills pay for the idle steps after a walk ends.
+constexpr int UNG_GROUP = 2;
 // QUEUE: a persistent grid whose lanes take hits from a grid-wide queue as their walks end (the
 // batched pipeline); otherwise one hit per thread, thread i taking hit i (the plain pipeline).
 template <bool QUEUE>
@@ -379,14 +377,14 @@ __global__ void __launch_bounds__(256) k_ungapped(DevLib L, DevQueries Q, const 
                                                    const unsigned int* __restrict__ n_list) {
     if (list) n = *n_list;  // the listed hits only
     __shared__ int32_t mat[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) mat[i] = P->matrix[i];
+    ung_table(mat, P->matrix);
     __syncthreads();
     const int32_t ws = P->word_size, xdrop = P->xdrop_ungap;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int phase = 0;  // 0 needs a hit, 1 walking, 3 queue empty
     uint64_t i = 0;
-    UngWalk walk;
+    UngBlocks walk;
     SeedHit h{0, 0};
     uint32_t lw = 0;
     bool taken = false;
@@ -428,7 +426,7 @@ __global__ void __launch_bounds__(256) k_ungapped(DevLib L, DevQueries Q, const 
         if (!__any_sync(FULL, phase == 1)) break;
 #pragma unroll
         for (int g = 0; g < UNG_GROUP; ++g) {
-            if (phase == 1 && walk.step(mat) == 2) {
+            if (phase == 1 && walk.step(mat)) {
                 // the box in the record frame, and the value the diagonal hash stores
                 int32_t sc;
                 uint32_t a, b, c, d;
@@ -592,6 +590,19 @@ __global__ void __launch_bounds__(256) k_bucket_leaders(uint64_t n, const uint32
 // together (a run of thousands of hits, a query against itself, waits for one batch after another).
 // SOME: only the hits with bit 31 have a box; an admitted one without is extended here.
 constexpr int REPLAY_BATCH = 8;
+// One extension, its box in the walk's frame.  Not inlined: the replay's batch would hold it eight times
+// (2.1 Mb against 2,000 consensi: 15.7 ms a launch inlined).
+__device__ __noinline__ UngBox walk_one(const int32_t* tab, const uint8_t* q, const uint8_t* s, int32_t qlen, int32_t slen,
+                                        int32_t seed_q, int32_t seed_s, int32_t xdrop) {
+    UngBlocks walk;
+    walk.start(q, s, qlen, slen, seed_q, seed_s, xdrop);
+    while (!walk.step(tab)) {
+    }
+    UngBox u{};
+    walk.result(u.score, u.q_start, u.q_end, u.s_start, u.s_end);
+    return u;
+}
+
 template <bool SOME>
 __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, const DevParams* __restrict__ P, int32_t ws,
                                                       int32_t ucut, uint64_t pair0, uint64_t n,
@@ -603,7 +614,7 @@ __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, co
                                                       uint8_t* __restrict__ flags, DiagCell* __restrict__ cells) {
     __shared__ int32_t mat[SOME ? 256 : 1];
     if (SOME) {
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) mat[i] = P->matrix[i];
+        ung_table(mat, P->matrix);
         __syncthreads();
     }
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -656,17 +667,12 @@ __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, co
                 const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
                 const uint32_t qlen = Q.len[qi], slen = L.len[si];
                 const SeedHit h = hits[i];
-                UngBox u;
-                uint32_t a, e, c, d;
-                UngWalk walk;
                 const int32_t qo = (int32_t)(h.qs & 0x7fffffffu), so = (int32_t)h.s;
-                const uint8_t* sp = L.plus + L.plus_off[si];
-                if (!(h.qs >> 31)) walk.start(Q.q + Q.off[qi], sp, (int32_t)qlen, (int32_t)slen, qo, so, P->xdrop_ungap);
-                else walk.start(Q.qrc + Q.off[qi], sp, (int32_t)qlen, (int32_t)slen, (int32_t)qlen - 1 - qo,
-                                (int32_t)slen - 1 - so, P->xdrop_ungap);
-                while (walk.step(mat) != 2) {
-                }
-                walk.result(u.score, a, e, c, d);
+                const bool minus = h.qs >> 31;
+                UngBox u = walk_one(mat, (minus ? Q.qrc : Q.q) + Q.off[qi], L.plus + L.plus_off[si], (int32_t)qlen,
+                                    (int32_t)slen, minus ? (int32_t)qlen - 1 - qo : qo,
+                                    minus ? (int32_t)slen - 1 - so : so, P->xdrop_ungap);
+                const uint32_t a = u.q_start, e = u.q_end, c = u.s_start, d = u.s_end;
                 if (!(h.qs >> 31)) {
                     u.q_start = a; u.q_end = e; u.s_start = c; u.s_end = d;
                     u.store = u.score >= ucut ? d : h.s + (uint32_t)ws;
@@ -714,7 +720,7 @@ __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, co
 // all search keeps ~1% of its hits), where extending every hit first wastes most of the work.
 constexpr int DDX_WARPS = 8;
 // a pass whose admitted hits are at most this many extends them one after another with the whole
-// warp (ung_walk_warp); more run one a lane (UngWalk)
+// warp (ung_walk_warp); more run one a lane (UngBlocks)
 constexpr int DDX_COOP = 6;
 // a hit-heavy pair's hits go to at most 2^DDX_GLOG_MAX bucket groups
 constexpr uint32_t DDX_GLOG_MAX = 5;
@@ -829,9 +835,10 @@ __global__ void __launch_bounds__(DDX_WARPS * 32, 4) k_dedup_extend(DevLib L, De
                                                                  DiagCell* __restrict__ cells,
                                                                  unsigned long long* __restrict__ queue,
                                                                  DedupUnits units) {
-    __shared__ int32_t mat[256];
+    __shared__ int32_t mat[256], tab[256];
     __shared__ uint32_t heads[DDX_WARPS][512];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) mat[i] = P->matrix[i];
+    ung_table(tab, P->matrix);
     __syncthreads();
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -949,11 +956,11 @@ __global__ void __launch_bounds__(DDX_WARPS * 32, 4) k_dedup_extend(DevLib L, De
                         }
                     } else if (ext) {
                         const int32_t qo = (int32_t)(h.qs & 0x7fffffffu), so = (int32_t)h.s;
-                        UngWalk walk;
+                        UngBlocks walk;
                         if (!(h.qs >> 31)) walk.start(qf, sp, (int32_t)qlen, (int32_t)slen, qo, so, xdrop);
                         else walk.start(qr, sp, (int32_t)qlen, (int32_t)slen, (int32_t)qlen - 1 - qo,
                                         (int32_t)slen - 1 - so, xdrop);
-                        while (walk.step(mat) != 2) {
+                        while (!walk.step(tab)) {
                         }
                         walk.result(sc, a0, a1, c0, c1);
                     }
