@@ -57,9 +57,9 @@ struct PairView {
 
 // engine.rs:1118-1149 (plus) and 1187-1218 (minus): exact extension to word_size on the
 // masked query; returns false if the word hit is dropped.  The two runs of matching bases beside the
-// word, at most ext_needed long, are counted in two plain loops over the whole warp (the sentinels at
-// the sequences' ends stop them), then limited in the strand's order: left first on the plus
-// strand, right first on the minus strand.  Early returns out of the loops are avoided on purpose:
+// word, at most ext_needed long, are counted in two loops of the whole warp (the sentinels at the
+// sequences' ends stop them; a loop ends when no lane's run goes on), then limited in the strand's
+// order: left first on the plus strand, right first on the minus strand.  Early returns out of the loops are avoided on purpose:
 // with them the warp was seen to reach the caller's vote in two parts (one hit in millions lost).
 __device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint32_t q0c, uint32_t p, uint32_t& qs,
                                              uint32_t& so) {
@@ -74,7 +74,7 @@ __device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint
     const uint8_t* s = (plus ? v.splus : v.src) + 1 + s0;
     int32_t left = 0, right = 0;
     bool on = there;
-    for (int32_t i = 0; i < need; ++i) {
+    for (int32_t i = 0; i < need && __any_sync(0xffffffffu, on); ++i) {
         uint8_t a = 15, b = 0;
         if (on) {
             a = q[-1 - i];
@@ -84,7 +84,7 @@ __device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint
         left += on;
     }
     on = there;
-    for (int32_t i = 0; i < need; ++i) {
+    for (int32_t i = 0; i < need && __any_sync(0xffffffffu, on); ++i) {
         uint8_t a = 15, b = 0;
         if (on) {
             a = q[v.lw + i];
@@ -125,8 +125,8 @@ __device__ __forceinline__ uint64_t scan_unit_of(const ScanUnits& U, uint32_t n_
 // Bound: the latency of a round's dependent loads (subject word, presence bit, cell start, cell entry,
 // query bytes).  So a round takes SCAN_POS positions a lane, their loads side by side, and its cells'
 // entries are spread over the warp as one list, one entry a lane.  Measured (B200) against one position a
-// lane and round: 1,000 contigs against 2,000 consensi (2 M pairs) 31 -> 18 ms, 120 chunks of 60 kb
-// 8.2 -> 3.3, 4,000 sequences at word 14 11.3 -> 8.2; and by stretches of pairs, 100 kb at word 7
+// lane and round: 1,000 contigs against 2,000 consensi (2 M pairs) 31 -> 14.7 ms, 120 chunks of 60 kb
+// 8.2 -> 2.8, 4,000 sequences at word 14 11.3 -> 6.0; and by stretches of pairs, 100 kb at word 7
 // 5.5 -> 0.1, 2.1 Mb against 2,000 consensi 50 -> 1.
 enum { SCAN_WRITE = 1, SCAN_STAGE = 2 };
 constexpr int SCAN_POS = 4;
