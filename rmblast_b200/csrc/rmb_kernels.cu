@@ -59,8 +59,9 @@ struct PairView {
 // masked query; returns false if the word hit is dropped.  The two runs of matching bases beside the
 // word, at most ext_needed long, are counted in two loops of the whole warp (the sentinels at the
 // sequences' ends stop them; a loop ends when no lane's run goes on), then limited in the strand's
-// order: left first on the plus strand, right first on the minus strand.  Early returns out of the loops are avoided on purpose:
-// with them the warp was seen to reach the caller's vote in two parts (one hit in millions lost).
+// order: left first on the plus strand, right first on the minus strand.  Early returns out of the
+// loops are avoided on purpose: with them the warp was seen to reach the caller's vote in two parts
+// (one hit in millions lost).
 __device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint32_t q0c, uint32_t p, uint32_t& qs,
                                              uint32_t& so) {
     const int64_t c1 = v.qlen + 1;
@@ -585,13 +586,24 @@ __global__ void __launch_bounds__(256) k_bucket_leaders(uint64_t n, const uint32
     }
 }
 
-// Thread k replays the run that starts at sorted hit k; its chain, oldest cell first, is
-// cells[k ..] with the newest cell in registers.  The hits come in batches whose loads go out
-// together (a run of thousands of hits, a query against itself, waits for one batch after another).
-// SOME: only the hits with bit 31 have a box; an admitted one without is extended here.
-constexpr int REPLAY_BATCH = 8;
-// One extension, its box in the walk's frame.  Not inlined: the replay's batch would hold it eight times
-// (2.1 Mb against 2,000 consensi: 15.7 ms a launch inlined).
+// The sorted hits that start a run, in no order.
+__global__ void __launch_bounds__(256) k_run_heads(uint64_t n, const uint32_t* __restrict__ keys,
+                                                   uint32_t* __restrict__ heads, unsigned int* __restrict__ n_heads) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t k0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; k0 < n; k0 += nwarps * 32) {
+        const uint64_t k = k0 + lane;
+        const bool head = k < n && (k == 0 || keys[k - 1] != keys[k]);
+        const unsigned m = __ballot_sync(0xffffffffu, head);
+        if (!m) continue;
+        unsigned int base = 0;
+        if (lane == 0) base = atomicAdd(n_heads, (unsigned)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (head) heads[base + __popc(m & ((1u << lane) - 1u))] = (uint32_t)k;
+    }
+}
+
+// One extension, its box in the walk's frame; not inlined, the replay's batch would hold it eight times.
 __device__ __noinline__ UngBox walk_one(const int32_t* tab, const uint8_t* q, const uint8_t* s, int32_t qlen, int32_t slen,
                                         int32_t seed_q, int32_t seed_s, int32_t xdrop) {
     UngBlocks walk;
@@ -603,6 +615,13 @@ __device__ __noinline__ UngBox walk_one(const int32_t* tab, const uint8_t* q, co
     return u;
 }
 
+// A thread replays the run that starts at sorted hit k; its chain, oldest cell first, is
+// cells[k ..] with the newest cell in registers.  The hits come in batches whose loads go out
+// together (a run of thousands of hits, a query against itself, waits for one batch after another).
+// SOME: only the hits with bit 31 have a box; an admitted one without is extended here, and the runs,
+// long and few, come from a list.  (With a thread a hit, all but the runs' first idle, a run held a
+// warp: 2.1 Mb against 50 consensi, 25,600 runs, took 15.6 ms, from the list 9.0.)
+constexpr int REPLAY_BATCH = 8;
 template <bool SOME>
 __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, const DevParams* __restrict__ P, int32_t ws,
                                                       int32_t ucut, uint64_t pair0, uint64_t n,
@@ -611,98 +630,103 @@ __global__ void __launch_bounds__(128) k_bucket_dedup(DevLib L, DevQueries Q, co
                                                       const int32_t* __restrict__ diags,
                                                       const uint32_t* __restrict__ hash_keys,
                                                       const SeedHit* __restrict__ hits, UngBox* __restrict__ ub,
-                                                      uint8_t* __restrict__ flags, DiagCell* __restrict__ cells) {
+                                                      uint8_t* __restrict__ flags, DiagCell* __restrict__ cells,
+                                                      const uint32_t* __restrict__ heads,
+                                                      const unsigned int* __restrict__ n_heads) {
     __shared__ int32_t mat[SOME ? 256 : 1];
     if (SOME) {
         ung_table(mat, P->matrix);
         __syncthreads();
     }
-    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t run = keys[k];
-    if (k > 0 && keys[k - 1] == run) return;
-    const int32_t window = 1 - ws;
-    DiagCell* pool = cells + k;
-    DiagCell head{0, 0, 0};
-    uint32_t m = 0;  // cells, the head included; the others are pool[0 .. m - 2]
-    bool more = true;
-    for (uint64_t j = k; more; j += REPLAY_BATCH) {
-        uint32_t bi[REPLAY_BATCH], bkey[REPLAY_BATCH], bstore[REPLAY_BATCH];
-        int32_t bdiag[REPLAY_BATCH], bscore[REPLAY_BATCH];
-        int cnt = 0;
+    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t end = SOME ? *n_heads : n;
+    for (uint64_t t = gid; t < end; t += stride) {
+        const uint64_t k = SOME ? heads[t] : t;
+        const uint32_t run = keys[k];
+        if (!SOME && k > 0 && keys[k - 1] == run) continue;
+        const int32_t window = 1 - ws;
+        DiagCell* pool = cells + k;
+        DiagCell head{0, 0, 0};
+        uint32_t m = 0;  // cells, the head included; the others are pool[0 .. m - 2]
+        bool more = true;
+        for (uint64_t j = k; more; j += REPLAY_BATCH) {
+            uint32_t bi[REPLAY_BATCH], bkey[REPLAY_BATCH], bstore[REPLAY_BATCH];
+            int32_t bdiag[REPLAY_BATCH], bscore[REPLAY_BATCH];
+            int cnt = 0;
 #pragma unroll
-        for (int b = 0; b < REPLAY_BATCH; ++b) {
-            const bool in = cnt == b && j + b < n && keys[j + b] == run;
-            cnt += in;
-            bi[b] = in ? vals[j + b] : 0;
-            bdiag[b] = in ? diags[j + b] : 0;
-            bkey[b] = in ? hash_keys[j + b] : 0;
-        }
-        more = cnt == REPLAY_BATCH;
+            for (int b = 0; b < REPLAY_BATCH; ++b) {
+                const bool in = cnt == b && j + b < n && keys[j + b] == run;
+                cnt += in;
+                bi[b] = in ? vals[j + b] : 0;
+                bdiag[b] = in ? diags[j + b] : 0;
+                bkey[b] = in ? hash_keys[j + b] : 0;
+            }
+            more = cnt == REPLAY_BATCH;
 #pragma unroll
-        for (int b = 0; b < REPLAY_BATCH; ++b)
-            if (b < cnt && (!SOME || bi[b] & LEAD)) {
-                bstore[b] = ub[bi[b] & ~LEAD].store;
-                bscore[b] = ub[bi[b] & ~LEAD].score;
-            }
+            for (int b = 0; b < REPLAY_BATCH; ++b)
+                if (b < cnt && (!SOME || bi[b] & LEAD)) {
+                    bstore[b] = ub[bi[b] & ~LEAD].store;
+                    bscore[b] = ub[bi[b] & ~LEAD].score;
+                }
 #pragma unroll
-        for (int b = 0; b < REPLAY_BATCH; ++b) {
-            if (b >= cnt) break;
-            const uint32_t i = bi[b] & ~LEAD, key = bkey[b];
-            const int32_t diag = bdiag[b];
-            uint32_t last = 0;
-            bool known = m > 0 && head.diag == diag;
-            if (known) last = head.level;
-            for (uint32_t c = m; !known && c > 1; --c)
-                if (pool[c - 2].diag == diag) {
-                    last = pool[c - 2].level;
-                    known = true;
+            for (int b = 0; b < REPLAY_BATCH; ++b) {
+                if (b >= cnt) break;
+                const uint32_t i = bi[b] & ~LEAD, key = bkey[b];
+                const int32_t diag = bdiag[b];
+                uint32_t last = 0;
+                bool known = m > 0 && head.diag == diag;
+                if (known) last = head.level;
+                for (uint32_t c = m; !known && c > 1; --c)
+                    if (pool[c - 2].diag == diag) {
+                        last = pool[c - 2].level;
+                        known = true;
+                    }
+                if (key < last) {
+                    flags[i] = 0;
+                    continue;
                 }
-            if (key < last) {
-                flags[i] = 0;
-                continue;
-            }
-            if (SOME && !(bi[b] & LEAD)) {
-                const uint64_t pair = pair0 + run / 512u;
-                const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
-                const uint32_t qlen = Q.len[qi], slen = L.len[si];
-                const SeedHit h = hits[i];
-                const int32_t qo = (int32_t)(h.qs & 0x7fffffffu), so = (int32_t)h.s;
-                const bool minus = h.qs >> 31;
-                UngBox u = walk_one(mat, (minus ? Q.qrc : Q.q) + Q.off[qi], L.plus + L.plus_off[si], (int32_t)qlen,
-                                    (int32_t)slen, minus ? (int32_t)qlen - 1 - qo : qo,
-                                    minus ? (int32_t)slen - 1 - so : so, P->xdrop_ungap);
-                const uint32_t a = u.q_start, e = u.q_end, c = u.s_start, d = u.s_end;
-                if (!(h.qs >> 31)) {
-                    u.q_start = a; u.q_end = e; u.s_start = c; u.s_end = d;
-                    u.store = u.score >= ucut ? d : h.s + (uint32_t)ws;
-                } else {
-                    u.q_start = qlen - e; u.q_end = qlen - a; u.s_start = slen - d; u.s_end = slen - c;
-                    u.store = u.score >= ucut ? d : key + (uint32_t)ws;
+                if (SOME && !(bi[b] & LEAD)) {
+                    const uint64_t pair = pair0 + run / 512u;
+                    const uint32_t qi = (uint32_t)(pair / L.n), si = (uint32_t)(pair % L.n);
+                    const uint32_t qlen = Q.len[qi], slen = L.len[si];
+                    const SeedHit h = hits[i];
+                    const int32_t qo = (int32_t)(h.qs & 0x7fffffffu), so = (int32_t)h.s;
+                    const bool minus = h.qs >> 31;
+                    UngBox u = walk_one(mat, (minus ? Q.qrc : Q.q) + Q.off[qi], L.plus + L.plus_off[si], (int32_t)qlen,
+                                        (int32_t)slen, minus ? (int32_t)qlen - 1 - qo : qo,
+                                        minus ? (int32_t)slen - 1 - so : so, P->xdrop_ungap);
+                    const uint32_t a = u.q_start, e = u.q_end, c = u.s_start, d = u.s_end;
+                    if (!(h.qs >> 31)) {
+                        u.q_start = a; u.q_end = e; u.s_start = c; u.s_end = d;
+                        u.store = u.score >= ucut ? d : h.s + (uint32_t)ws;
+                    } else {
+                        u.q_start = qlen - e; u.q_end = qlen - a; u.s_start = slen - d; u.s_end = slen - c;
+                        u.store = u.score >= ucut ? d : key + (uint32_t)ws;
+                    }
+                    ub[i] = u;
+                    bstore[b] = u.store;
+                    bscore[b] = u.score;
                 }
-                ub[i] = u;
-                bstore[b] = u.store;
-                bscore[b] = u.score;
-            }
-            flags[i] = bscore[b] >= ucut ? 3 : 1;
-            if (m > 0 && (head.diag == diag || (int32_t)(key - head.level) > window)) {
-                head.diag = diag;
-                head.level = bstore[b];
-                continue;
-            }
-            bool done = false;
-            for (uint32_t c = m; !done && c > 1; --c) {
-                DiagCell& cl = pool[c - 2];
-                if (cl.diag == diag || (int32_t)(key - cl.level) > window) {
-                    cl.diag = diag;
-                    cl.level = bstore[b];
-                    done = true;
+                flags[i] = bscore[b] >= ucut ? 3 : 1;
+                if (m > 0 && (head.diag == diag || (int32_t)(key - head.level) > window)) {
+                    head.diag = diag;
+                    head.level = bstore[b];
+                    continue;
                 }
-            }
-            if (!done) {
-                if (m > 0) pool[m - 1] = head;
-                head = DiagCell{diag, bstore[b], 0};
-                ++m;
+                bool done = false;
+                for (uint32_t c = m; !done && c > 1; --c) {
+                    DiagCell& cl = pool[c - 2];
+                    if (cl.diag == diag || (int32_t)(key - cl.level) > window) {
+                        cl.diag = diag;
+                        cl.level = bstore[b];
+                        done = true;
+                    }
+                }
+                if (!done) {
+                    if (m > 0) pool[m - 1] = head;
+                    head = DiagCell{diag, bstore[b], 0};
+                    ++m;
+                }
             }
         }
     }
@@ -2664,11 +2688,15 @@ cudaError_t launch_bucket_dedup(const DevLib& L, const DevQueries& Q, const DevP
         if (e != cudaSuccess) return e;
         e = launch_ungapped(L, Q, P, ucut, n, hits, hit_pair, ub, sms, st, queue, blocks_per_sm, lead, n_lead);
         if (e != cudaSuccess) return e;
-        k_bucket_dedup<true><<<runs, 128, 0, st>>>(L, Q, P, ws, ucut, pair0, n, keys2, vals2, diags, hash_keys, hits, ub,
-                                                   flags, (DiagCell*)cells);
+        // the walks have read the list and its count
+        e = cudaMemsetAsync(n_lead, 0, 4, st);
+        if (e != cudaSuccess) return e;
+        k_run_heads<<<grid, 256, 0, st>>>(n, keys2, lead, n_lead);
+        k_bucket_dedup<true><<<std::min<unsigned>(2 * runs, 32 * (unsigned)sms), 64, 0, st>>>(
+            L, Q, P, ws, ucut, pair0, n, keys2, vals2, diags, hash_keys, hits, ub, flags, (DiagCell*)cells, lead, n_lead);
     } else {
         k_bucket_dedup<false><<<runs, 128, 0, st>>>(L, Q, P, ws, ucut, pair0, n, keys2, vals2, diags, hash_keys, hits, ub,
-                                                    flags, (DiagCell*)cells);
+                                                    flags, (DiagCell*)cells, nullptr, nullptr);
     }
     return cudaGetLastError();
 }
