@@ -395,7 +395,7 @@ class Results:
         _check(lib().rmb_format_tabular(self._s._ctx, self._p, ids, outfmt.encode(), C.byref(txt), C.byref(n), err,
                                         512), err)
         try:
-            return C.string_at(txt.value, n.value).decode()
+            return str((C.c_char * n.value).from_address(txt.value), "utf-8")  # no copy as bytes between
         finally:
             lib().rmb_text_free(txt)
 

@@ -455,9 +455,9 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     const rmb_tune& tn = C.tune;
     // The bucket replay, of all hits extended first or, in dense ranges, of the leaders.  k_dedup_extend
     // keeps the dense ranges whose pairs hold few thousand hits: it extends no dropped hit, and a warp a
-    // pair is enough lanes there (50 queries of 5 kb against 300 of their own, 4,700 hits a pair: 21 ms
-    // to 27); over 8,192 hits a pair its rounds wait on one pair's buckets (100 kb against 50 consensi,
-    // 31,000 hits a pair: 10.6 ms to 0.9; two of 60 kb against 2,000, 20,000: 51 to 34).
+    // pair is enough lanes there (40 consensi of 5 kb against their 1,000, 3,500 hits a pair: 20 ms to
+    // 34); over 8,192 hits a pair its rounds wait on one pair's buckets (100 kb against 50 consensi,
+    // 31,000 hits a pair: 10.6 ms to 0.7; 2.1 Mb against 50: 129 to 14).
     const bool bucket_fits = bucket_dedup_fits(npairs, nh);
     const bool leaders = fused && bucket_fits && nh >= (uint64_t)BUCKET_DENSE_HITS * npairs;
     const bool buckets = bucket_fits && (leaders || !fused);
@@ -2477,34 +2477,52 @@ int rmb_format_tabular(const rmb_ctx* C, const rmb_results* R, const char* const
         if (t != "6") throw Fail(RMB_EINVAL, "output format '" + t + "' is not supported; use 6 <fields>");
         while (is >> t) fields.push_back(t);
         if (fields.empty()) throw Fail(RMB_EINVAL, "-outfmt 6 needs a field list");
-        // queries formatted in parallel, each into its own string, then joined in query order
-        for (uint32_t qi = 0; qi < R->n_queries; ++qi)
-            for (uint64_t k = R->query_off[qi]; k < R->query_off[qi + 1]; ++k)
+        std::vector<uint8_t> ids;
+        if (!tabular_fields(fields, ids) && R->n_queries && R->query_off[R->n_queries])
+            throw Fail(RMB_EINVAL, "unknown -outfmt field");
+        // pieces of a query's lines, about 64 kB each, formatted in parallel and joined in order (a piece
+        // a query left one query's text, 5 ms of a 2.1 Mb search, to one core)
+        struct Piece {
+            uint32_t query;
+            uint64_t begin, end;
+            size_t bytes;
+        };
+        std::vector<Piece> pieces;
+        for (uint32_t qi = 0; qi < R->n_queries; ++qi) {
+            Piece p{qi, R->query_off[qi], R->query_off[qi], 0};
+            for (uint64_t k = p.begin; k < R->query_off[qi + 1]; ++k) {
                 if (R->hsps[k].subject_oid >= C->ids.size()) throw Fail(RMB_EINVAL, "HSP subject out of range");
-        std::vector<std::string> parts(R->n_queries);
-        std::atomic<bool> unknown{false};
-        parallel_for(R->n_queries, [&](size_t qi) {
-            const std::string qid = query_ids ? query_ids[qi] : ("query" + std::to_string(qi));
-            std::string& o = parts[qi];
+                p.bytes += 2 * (size_t)R->hsps[k].aln_len + 160;
+                p.end = k + 1;
+                if (p.bytes < 65536 && p.end < R->query_off[qi + 1]) continue;
+                pieces.push_back(p);
+                p = Piece{qi, p.end, p.end, 0};
+            }
+        }
+        std::vector<std::string> parts(pieces.size());
+        parallel_for(pieces.size(), [&](size_t i) {
+            const Piece& p = pieces[i];
+            const std::string qid = query_ids ? query_ids[p.query] : ("query" + std::to_string(p.query));
+            parts[i].reserve(p.bytes);
             Hit h;
-            for (uint64_t k = R->query_off[qi]; k < R->query_off[qi + 1] && !unknown; ++k) {
+            for (uint64_t k = p.begin; k < p.end; ++k) {
                 hit_from_record(R, k, h);
-                if (!format_line(o, h, qid, C->ids[R->hsps[k].subject_oid], fields)) unknown = true;
-                o.push_back('\n');
+                format_line(parts[i], h, qid, C->ids[R->hsps[k].subject_oid], ids);
+                parts[i].push_back('\n');
             }
         });
-        if (unknown) throw Fail(RMB_EINVAL, "unknown -outfmt field");
-        size_t total = 0;
-        for (const auto& x : parts) total += x.size();
-        std::string out;
-        out.reserve(total);
-        for (const auto& x : parts) out += x;
-        char* o = (char*)malloc(out.size() + 1);
+        std::vector<size_t> at(parts.size() + 1, 0);
+        for (size_t i = 0; i < parts.size(); ++i) at[i + 1] = at[i] + parts[i].size();
+        const size_t total = at.back();
+        char* o = (char*)malloc(total + 1);
         if (!o) throw std::bad_alloc();
-        memcpy(o, out.data(), out.size());
-        o[out.size()] = 0;
+        if (total > (4u << 20))
+            parallel_for(parts.size(), [&](size_t i) { memcpy(o + at[i], parts[i].data(), parts[i].size()); });
+        else
+            for (size_t i = 0; i < parts.size(); ++i) memcpy(o + at[i], parts[i].data(), parts[i].size());
+        o[total] = 0;
         *text = o;
-        if (text_len) *text_len = out.size();
+        if (text_len) *text_len = total;
         return RMB_OK;
     } catch (const Fail& e) {
         return fail_out(e, err, errlen, e.code);

@@ -2,9 +2,11 @@
 #include "rmb_glue.hpp"
 
 #include <algorithm>
+#include <charconv>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <map>
 #include <strings.h>
 
@@ -879,39 +881,82 @@ void sort_hit_list_order(std::vector<Hit>& r, const std::vector<std::string>& id
     });
 }
 
-bool format_line(std::string& out, const Hit& h, const std::string& qid, const std::string& sid,
-                 const std::vector<std::string>& fields) {
-    char buf[64];
-    const uint32_t s1 = h.s_start + 1, se = h.s_end;
-    bool first = true;
-    for (const std::string& f : fields) {
-        if (!first) out.push_back('\t');
-        first = false;
-        if (f == "score") out += std::to_string(h.score);
-        else if (f == "perc_sub") { snprintf(buf, sizeof buf, "%.2f", (double)h.stats.perc_sub); out += buf; }
-        else if (f == "perc_query_gap") { snprintf(buf, sizeof buf, "%.2f", (double)h.stats.perc_query_gap); out += buf; }
-        else if (f == "perc_db_gap") { snprintf(buf, sizeof buf, "%.2f", (double)h.stats.perc_db_gap); out += buf; }
-        else if (f == "qseqid") out += qid;
-        else if (f == "qstart") out += std::to_string(h.q_start + 1);
-        else if (f == "qend") out += std::to_string(h.q_end);
-        else if (f == "qlen") out += std::to_string(h.q_len);
-        else if (f == "sstrand") out += h.strand == 0 ? "plus" : "minus";
-        else if (f == "sseqid") out += sid;
-        else if (f == "sstart") out += std::to_string(h.strand == 0 ? s1 : se);
-        else if (f == "send") out += std::to_string(h.strand == 0 ? se : s1);
-        else if (f == "slen") out += std::to_string(h.s_len);
-        else if (f == "kdiv") { snprintf(buf, sizeof buf, "%.2f", h.stats.kdiv); out += buf; }
-        else if (f == "cpg_kdiv") { snprintf(buf, sizeof buf, "%.2f", h.stats.cpg_kdiv); out += buf; }
-        else if (f == "transi") out += std::to_string(h.stats.transversions);  // output.rs:160-164
-        else if (f == "transv") out += std::to_string(h.stats.cpg_sites);
-        else if (f == "cpg_sites") out += std::to_string(h.stats.transitions);
-        else if (f == "qseq") for (uint8_t b : h.q_seq) out.push_back(b == 15 ? '-' : IUPAC[b & 15]);
-        else if (f == "sseq") for (uint8_t b : h.s_seq) out.push_back(b == 15 ? '-' : IUPAC[b & 15]);
-        else if (f == "evalue") append_evalue(out, h.evalue);
-        else if (f == "bitscore") append_bitscore(out, h.bitscore);
-        else return false;
+bool tabular_fields(const std::vector<std::string>& names, std::vector<uint8_t>& fields) {
+    static const char* const NAMES[] = {"score",  "perc_sub", "perc_query_gap", "perc_db_gap", "qseqid", "qstart", "qend",
+                                        "qlen",   "sstrand",  "sseqid",         "sstart",      "send",   "slen",   "kdiv",
+                                        "cpg_kdiv", "transi", "transv",         "cpg_sites",   "qseq",   "sseq",   "evalue",
+                                        "bitscore"};
+    fields.clear();
+    for (const std::string& n : names) {
+        size_t k = 0;
+        while (k < std::size(NAMES) && n != NAMES[k]) ++k;
+        if (k == std::size(NAMES)) return false;
+        fields.push_back((uint8_t)k);
     }
     return true;
+}
+
+static void append_int(std::string& out, int64_t v) {
+    char buf[24];
+    out.append(buf, std::to_chars(buf, buf + sizeof buf, v).ptr);
+}
+// "%.2f": the nearest hundredth from the product, unless the product lies close to a tie
+static void append_fixed2(std::string& out, double v) {
+    char buf[64];
+    if (v >= 0.0 && v < 1e9 && !std::signbit(v)) {
+        const double r = v * 100.0;  // off by 1.2e-5 at most
+        uint64_t n = (uint64_t)r;
+        const double part = r - (double)n;
+        if (std::fabs(part - 0.5) > 1e-4) {
+            n += part > 0.5;
+            append_int(out, (int64_t)(n / 100));
+            const char frac[3] = {'.', (char)('0' + n / 10 % 10), (char)('0' + n % 10)};
+            out.append(frac, 3);
+            return;
+        }
+    }
+    snprintf(buf, sizeof buf, "%.2f", v);
+    out += buf;
+}
+static void append_bases(std::string& out, const std::vector<uint8_t>& seq) {
+    const size_t n = out.size();
+    out.resize(n + seq.size());
+    char* o = &out[n];
+    for (size_t i = 0; i < seq.size(); ++i) o[i] = IUPAC[seq[i] & 15];  // 15, a gap, is IUPAC's '-'
+}
+
+void format_line(std::string& out, const Hit& h, const std::string& qid, const std::string& sid,
+                 const std::vector<uint8_t>& fields) {
+    const uint32_t s1 = h.s_start + 1, se = h.s_end;
+    bool first = true;
+    for (const uint8_t f : fields) {
+        if (!first) out.push_back('\t');
+        first = false;
+        switch (f) {
+        case 0: append_int(out, h.score); break;
+        case 1: append_fixed2(out, (double)h.stats.perc_sub); break;
+        case 2: append_fixed2(out, (double)h.stats.perc_query_gap); break;
+        case 3: append_fixed2(out, (double)h.stats.perc_db_gap); break;
+        case 4: out += qid; break;
+        case 5: append_int(out, h.q_start + 1); break;
+        case 6: append_int(out, h.q_end); break;
+        case 7: append_int(out, h.q_len); break;
+        case 8: out += h.strand == 0 ? "plus" : "minus"; break;
+        case 9: out += sid; break;
+        case 10: append_int(out, h.strand == 0 ? s1 : se); break;
+        case 11: append_int(out, h.strand == 0 ? se : s1); break;
+        case 12: append_int(out, h.s_len); break;
+        case 13: append_fixed2(out, h.stats.kdiv); break;
+        case 14: append_fixed2(out, h.stats.cpg_kdiv); break;
+        case 15: append_int(out, h.stats.transversions); break;  // output.rs:160-164
+        case 16: append_int(out, h.stats.cpg_sites); break;
+        case 17: append_int(out, h.stats.transitions); break;
+        case 18: append_bases(out, h.q_seq); break;
+        case 19: append_bases(out, h.s_seq); break;
+        case 20: append_evalue(out, h.evalue); break;
+        default: append_bitscore(out, h.bitscore);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -88,9 +88,11 @@ void sort_prelims_for_traceback(std::vector<Prelim>& p, uint32_t qa, uint32_t sa
 void apply_mask_level(std::vector<Hit>& hits, uint32_t mask_level);
 void sort_hit_list_order(std::vector<Hit>& hits, const std::vector<std::string>& subject_ids);
 
-// output.rs:294-367 one tabular line (no newline); returns false on an unknown field.
-bool format_line(std::string& out, const Hit& h, const std::string& qid, const std::string& sid,
-                 const std::vector<std::string>& fields);
+// output.rs:294-367: the numbers of a tabular line's fields (false: an unknown one), and one line of them
+// (no newline).
+bool tabular_fields(const std::vector<std::string>& names, std::vector<uint8_t>& fields);
+void format_line(std::string& out, const Hit& h, const std::string& qid, const std::string& sid,
+                 const std::vector<uint8_t>& fields);
 
 int choose_lut_width(int word_size, uint64_t approx_entries);
 
