@@ -41,11 +41,11 @@ sys.path.insert(0, str(ROOT))
 
 FIELDS = "6 score perc_sub qseqid qstart qend sseqid sstart send"
 OPS_PER_CELL = 11  # int32 add/sub/max/compare per DP cell in search/gapped.rs:234-262
-# DRAM bytes (read + write) per ungapped record of k_prelim_stream, from one ncu capture of
-# `bench.py --workload plain --scale 0.01` (1.31 M records, 80.1 MB); the traffic is per record
-# (the 48-byte geometry read, the 28-byte result write, sequence words), so a launch's traffic
-# is this times its records
-PRELIM_STREAM_DRAM_BYTES_PER_RECORD = 61.0
+# DRAM bytes (read + write) per ungapped record of the preliminary DP, from one ncu capture of the
+# kernel's int32 form on `bench.py --workload plain --scale 0.01` (1.31 M records, 80.1 MB); the
+# traffic is per record (the 48-byte geometry read, the 28-byte result write, sequence words), the
+# same in the packed form, so a launch's traffic is this times its records
+PRELIM_DRAM_BYTES_PER_RECORD = 61.0
 # copy bandwidth of this pool's B200s measured earlier, used when MEASURED_PEAKS.json is absent
 HBM_FALLBACK_GBS = 6650.0
 BATCH_CHUNKS = 1000
@@ -411,13 +411,14 @@ def main():
     k = kernel_pass(s) if args.pipeline == "batched" else c
     prelim_ms = k["gpu_ms_prelim"]
     so_cells = k["so_cells"]
-    # the dominant kernel: k_prelim_stream (one launch per sub-batch), timed alone with CUDA events
+    # the dominant kernels: the preliminary DP's (k_prelim_dual and the records it lists, or, where the scores
+    # do not fit the packed rows, k_prelim_stream), timed alone with CUDA events
     main_ms, main_cells = k["gpu_ms_prelim_main"], k["so_cells_main"]
     if main_ms <= 0:  # parameters outside the thread kernel's range: the warp kernel does it all
         main_ms, main_cells = prelim_ms, so_cells
     achieved = main_cells * OPS_PER_CELL / (main_ms * 1e-3) / 1e12 if main_ms > 0 else 0.0
-    traffic = (PRELIM_STREAM_DRAM_BYTES_PER_RECORD * k["prelim_dp"]
-               if PRELIM_STREAM_DRAM_BYTES_PER_RECORD and k["gpu_ms_prelim_main"] > 0 else None)
+    traffic = (PRELIM_DRAM_BYTES_PER_RECORD * k["prelim_dp"]
+               if PRELIM_DRAM_BYTES_PER_RECORD and k["gpu_ms_prelim_main"] > 0 else None)
     peaks, peak_source = {"hbm_gbs": HBM_FALLBACK_GBS}, "fallback"
     pk = ROOT / "MEASURED_PEAKS.json"
     if pk.exists():
@@ -445,7 +446,7 @@ def main():
                                                  "ms_host_2a", "ms_traceback", "ms_host_2b")},
         "counts": {k: int(c[k]) for k in ("word_hits", "ungapped", "prelim_dp", "prelims", "tb_dp", "finals",
                                           "so_cells", "tb_cells")},
-        "roofline": {"kernel": "k_prelim_stream (score-only X-drop DP)", "bound": "int32", "achieved": achieved,
+        "roofline": {"kernel": "k_prelim_dual + k_prelim_pack (score-only X-drop DP)", "bound": "int32", "achieved": achieved,
                      "peak": peak_int, "unit": "Tops/s", "frac": achieved / peak_int if peak_int else None,
                      "traffic": traffic, "kernel_ms": main_ms, "cells": main_cells,
                      "hbm": {"achieved_gbs": traffic / (main_ms * 1e-3) / 1e9 if traffic else None,
@@ -453,9 +454,10 @@ def main():
                              "frac": (traffic / (main_ms * 1e-3) / 1e9 / peaks["hbm_gbs"]
                                       if traffic and peaks.get("hbm_gbs") else None)},
                      "note": f"{OPS_PER_CELL} int32 ops per DP cell (the reference's cell step) x cells of the "
-                             "records k_prelim_stream completed / its event time; peak = rmb_probe_int32_peak "
-                             "(dependent int32 add/max throughput of this GPU) measured in this run; the kernel "
-                             "is bound by integer issue, not by HBM (hbm.frac) or tensor cores"},
+                             "records these kernels completed / their event time (they take two cells an "
+                             "operation, in 16-bit halves); peak = rmb_probe_int32_peak "
+                             "(dependent int32 add/max throughput of this GPU) measured in this run; the kernels "
+                             "are bound by integer issue, not by HBM (hbm.frac) or tensor cores"},
         "gpu_launches": int(c["launches"] * args.steps),
         "clocks": clk,
         "e2e": {"value": timed_bases * world / (e2e_ms * 1e-3) / 1e6, "unit": "Mbp/s",

@@ -2,20 +2,22 @@
 //
 //   k_scan        lookup-table scan of the packed library + exact word extension
 //                 (blast/nascan.rs, blast/mblookup.rs:247-343, engine.rs:1118-1218); a warp per
-//                 (query, subject) pair, lanes on consecutive scan offsets, two passes (count,
-//                 then write at the pair's prefix offset) so every pair's hits keep scan order.
-//   k_ungapped    ungapped X-drop extension of every word hit (search/ungapped.rs:38-121),
-//                 one thread per hit, computed for all hits ahead of the dedup.
-//   k_dedup       the order-dependent diagonal hash (search/diag_hash.rs) replayed per pair in
-//                 scan order on the precomputed extensions, one thread per pair.
-//   k_prelim_warp preliminary score-only X-drop DP (search/gapped.rs:124-418) of every ungapped
-//                 record, one warp per record, the DP band in a shared-memory ring;
-//                 k_prelim_wide reruns the records whose band outgrew the ring with the band in
-//                 global memory (one thread per record).
-//   k_traceback_warp  improve_seed + traceback X-drop DP + trace walk (engine.rs:383-572,
-//                 engine.rs:2953-3039, search/gapped.rs:450-757), one warp per prelim HSP.
+//                 (query, subject) pair or stretch of one, four scan offsets a lane, hits staged in
+//                 scan order and gathered into pair order.
+//   k_ungapped    ungapped X-drop extension of word hits (search/ungapped.rs:38-121), a walk a lane
+//                 eight bases a step.
+//   k_bucket_dedup, k_dedup_extend, k_dedup  the order-dependent diagonal hash (search/diag_hash.rs)
+//                 replayed in scan order: a thread per (pair, bucket) run of sorted hits; a warp per
+//                 pair with the extension of admitted hits; a thread per pair (the plain pipeline).
+//   k_prelim_dual, k_prelim_pack  preliminary score-only X-drop DP (search/gapped.rs:124-418) in packed
+//                 16-bit rows: two records a thread, then 8 lanes an extension for the records that
+//                 reach the cutoff or outgrow the window; k_prelim_stream where the scores do not fit;
+//                 k_prelim_warp_dir and k_prelim_wide for bands that outgrow those.
+//   k_traceback_pack, k_traceback_warp  improve_seed + traceback X-drop DP + trace walk
+//                 (engine.rs:383-572, engine.rs:2953-3039, search/gapped.rs:450-757), a warp per
+//                 extension, the band in registers; or in memory for what does not fit.
 //
-// All scores are int32; the arithmetic and the order of every comparison follow the cited
+// All scores are integers; the arithmetic and the order of every comparison follow the cited
 // reference functions so results are bit-identical.
 #include <algorithm>
 #include <cstdint>
