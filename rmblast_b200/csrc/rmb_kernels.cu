@@ -306,65 +306,10 @@ __global__ void __launch_bounds__(256) k_scan_gather(ScanUnits U, uint32_t n_sub
 // ---------------------------------------------------------------------------------------
 // ungapped extension: search/ungapped.rs:38-121
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void extend_ungapped(const uint8_t* query, int64_t q_real, const uint8_t* subject,
-                                                int64_t s_real, uint32_t q_off, uint32_t s_off, const int32_t* mat,
-                                                int32_t xdrop, int32_t& score_out, uint32_t& qs_out, uint32_t& qe_out,
-                                                uint32_t& ss_out, uint32_t& se_out) {
-    const int32_t x = -xdrop;
-    const int64_t qo = q_off, so = s_off;
-    int32_t score = 0, sum = 0;
-    int64_t q_beg = qo;
-    {
-        int64_t q = qo - 1, s = so - 1;
-        while (q >= 0 && s >= 0) {
-            const uint8_t qb = query[1 + q], sb = subject[1 + s];
-            if (qb == 15 || sb == 15) break;
-            sum += mat[((qb & 15) << 4) | (sb & 15)];
-            if (sum > 0) {
-                q_beg = q;
-                score += sum;
-                sum = 0;
-            } else if (sum < x) {
-                break;
-            }
-            --q;
-            --s;
-        }
-    }
-    int64_t q_end = qo;
-    int32_t xc = x;
-    sum = 0;
-    {
-        int64_t q = qo, s = so;
-        while (q < q_real && s < s_real) {
-            const uint8_t qb = query[1 + q], sb = subject[1 + s];
-            if (qb == 15 || sb == 15) break;
-            sum += mat[((qb & 15) << 4) | (sb & 15)];
-            if (sum > 0) {
-                q_end = q + 1;
-                score += sum;
-                xc = (-score > x) ? -score : x;
-                sum = 0;
-            } else if (sum < xc) {
-                break;
-            }
-            ++q;
-            ++s;
-        }
-    }
-    score_out = score;
-    qs_out = (uint32_t)q_beg;
-    qe_out = (uint32_t)q_end;
-    ss_out = (uint32_t)(so - (qo - q_beg));
-    se_out = (uint32_t)(so + (q_end - qo));
-}
-
-// engine.rs:1165-1170 (plus) and 1244-1261 (minus): the extension in NCBI's frame, its box in
-// the record frame, and the value the diagonal hash stores for the seed.
-// One word hit per lane at a time: the two walks of extend_ungapped (left, then right, in the
+// One word hit per lane at a time: the two walks of an extension (left, then right, in the
 // strand's frame) as one resumable walk of UNG_GROUP steps per round; a lane whose hit is done
 // takes the next hit index from the grid-wide queue (one atomic per warp and round), so lanes do
-// not wait for the longest walk of the warp.  Same arithmetic as extend_ungapped + the box of
+// not wait for the longest walk of the warp.  The reference's arithmetic, and the box of
 // engine.rs:1165-1170 / 1244-1261.
 // UNG_GROUP steps of eight bases a round: the walks at the default size run hundreds of bases, so
 // fewer refills pay for the idle steps after a walk ends.
