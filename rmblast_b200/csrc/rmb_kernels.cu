@@ -3020,8 +3020,10 @@ bool traceback_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t
     const int32_t goe = gap_open + gap_extend, xmax = std::max(xdrop, goe);
     if (gap_extend < 1 || gap_extend > 40 || gap_open < 0 || xmax > 4000) return false;
     if ((xmax - goe) / gap_extend + 1 + TB_K >= TB_W - 1) return false;
+    // a dead cell is 0 and the lowest live value, one X below a best of 0 in the first row, TB_LIVE + 2 gap_extend
+    // on the first window diagonal: a score with its decay has to stay below it
     for (int i = 0; i < 256; ++i)
-        if (matrix256[i] > 2000) return false;
+        if (matrix256[i] >= TB_LIVE) return false;
     return true;
 }
 

@@ -5,10 +5,11 @@
 // The rows are k_prelim_pack's (rmb_prelim_pack.cuh: window of diagonals, packed 16-bit values,
 // coordinates, exactness), with the whole warp on one extension, TB_W = 128 diagonals, four a lane.  The
 // scores are 16-bit table entries (two byte lookups and a merge), so the X-drop is limited by the
-// window alone.  A cell's trace is four bits: the vertical gap beat the diagonal, the horizontal gap beat
-// both, and either gap's extension is at least its opening, gapped.rs:577-618's op byte; a row's 128 are
-// 64 bytes, one 16-bit store a lane, with the row's window position beside them.  On cells below the
-// X-drop threshold they may differ from the reference's, and no path visits those.
+// window alone, and the scores by what keeps a dead cell dead (TB_LIVE).  A cell's trace is four bits:
+// the vertical gap beat the diagonal, the horizontal gap beat both, and either gap's extension is at
+// least its opening, gapped.rs:577-618's op byte; a row's 128 are 64 bytes, one 16-bit store a lane,
+// with the row's window position beside them.  On cells below the X-drop threshold they may differ
+// from the reference's, and no path visits those.
 //
 // The walk goes by runs: lane l looks at the cell l steps up the path's diagonal, and the warp takes the
 // run of substitutions to the first gap, 32 at most, at once; a gap's cells go one by one.
@@ -22,6 +23,7 @@ namespace rmb {
 constexpr int TB_R = 2, TB_W = 64 * TB_R, TB_K = TB_W / 2 - 2;
 constexpr uint32_t TB_ROW_BYTES = TB_W / 2 + 4;  // trace and window position of a row
 constexpr int32_t TB_SCORE_MIN = -8192;          // a blocked column's score: ends any path
+constexpr int32_t TB_LIVE = 256;                 // live values stay above it: no score of a cell reaches it
 
 // Status of an extension that its window or its codes do not fit: the byte-trace kernel takes it.
 constexpr int TB_WIDE = 4;
@@ -55,7 +57,7 @@ __device__ __forceinline__ int tb_pack_extend(const uint8_t* __restrict__ a, con
     auto code_at = [&](int32_t j) -> uint32_t { return j < 0 ? 0u : j >= n ? 5u : tb_code(b[(ptrdiff_t)dir * j]); };
 
     uint32_t H[R], E[R], sel[R], S[R];
-    int32_t bo = X + 256, k0 = -TB_K, best = 0, best_bo = 0, best_k0 = 0, row = 0;
+    int32_t bo = X + TB_LIVE, k0 = -TB_K, best = 0, best_bo = 0, best_k0 = 0, row = 0;
     uint32_t best_a = 0;
     cells = (uint64_t)J + 1;
     bool odd = false;
