@@ -213,7 +213,8 @@ int rmb_search_batch(rmb_ctx* ctx, uint32_t n_queries, const uint8_t* const* que
 /* The same search split at the host/device boundary: rmb_queries_upload copies the queries
  * into device memory once (the reference's per-query BLASTNA buffers, main.rs:740-746), and
  * rmb_search_resident runs search_db_parallel on them; rmb_search_batch is upload + search +
- * free.  A query set belongs to the device of the context that uploaded it. */
+ * free.  A query set belongs to the device of the context that uploaded it; several contexts on that
+ * device may search it, also at the same time (it must not be freed meanwhile). */
 typedef struct rmb_queries rmb_queries;
 int rmb_queries_upload(rmb_ctx* ctx, uint32_t n_queries, const uint8_t* const* query, const uint32_t* qlen,
                        rmb_queries** out, char* err, size_t errlen);

@@ -259,9 +259,12 @@ struct rmb_queries {
     std::vector<uint64_t> off;     // offset of query i in host / d_q / d_qrc
     std::vector<uint32_t> len;
     DBuf d_q, d_qrc, d_off, d_len;
-    DBuf d_qm, d_qmrc;   // DUST-masked queries and their reverse complements (made on first use)
+    // Made by the first search that needs them, under `mu`: contexts on several host threads may search
+    // one set.  A flag goes up when the device has finished the copies it stands for.
+    std::mutex mu;
+    DBuf d_qm, d_qmrc;   // DUST-masked queries and their reverse complements
     bool dusted = false;
-    DBuf d_dp;           // the packed-row DP's copies (made on first use)
+    DBuf d_dp;           // the packed-row DP's copies
     uint64_t dp_stride = 0;
     bool dp_made = false;
     void release() {
@@ -720,13 +723,17 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
     }
     cudaStream_t st = C.st;
     upload(C.lw, lw_all, st);
-    if (P.dust && !QH.dusted && nq) mask_queries(C, QH, false, ctr);
-    if (C.prelim_pack && !QH.dp_made && nq) {
-        QH.dp_stride = dp_query_stride(QH.host.size(), nq);
-        QH.d_dp.ensure(dp_bytes(4, QH.dp_stride));
-        CK(launch_dp_query(QH.d_q.as<uint8_t>(), QH.d_qrc.as<uint8_t>(), QH.d_off.as<uint64_t>(),
-                           QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride, st));
-        QH.dp_made = true;
+    if (nq) {
+        std::lock_guard<std::mutex> lock(QH.mu);
+        if (P.dust && !QH.dusted) mask_queries(C, QH, false, ctr);
+        if (C.prelim_pack && !QH.dp_made) {
+            QH.dp_stride = dp_query_stride(QH.host.size(), nq);
+            QH.d_dp.ensure(dp_bytes(4, QH.dp_stride));
+            CK(launch_dp_query(QH.d_q.as<uint8_t>(), QH.d_qrc.as<uint8_t>(), QH.d_off.as<uint64_t>(),
+                               QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride, st));
+            CK(cudaStreamSynchronize(st));
+            QH.dp_made = true;
+        }
     }
     const uint8_t* qmask = P.dust ? QH.d_qm.as<uint8_t>() : QH.d_q.as<uint8_t>();
     const uint8_t* qmask_rc = P.dust ? QH.d_qmrc.as<uint8_t>() : QH.d_qrc.as<uint8_t>();
