@@ -69,7 +69,8 @@ typedef struct rmb_ctx rmb_ctx;
  * rmb_autotune times candidates on sample queries and keeps the fastest; rmb_tune_get/set read
  * and write them (a caller can persist and reuse a tuned set).
  * The prelim_* knobs but prelim_window shape the thread-per-extension DP, which runs where the
- * packed-row DP's number ranges do not hold (an X-drop over 128, scores near 127).
+ * packed-row DP's number ranges do not hold (an X-drop over 128, scores near 127) and where many of a
+ * large search's records meet ambiguity codes other than N.
  *   prelim_group            cell steps a lane of the thread-per-extension DP runs between its
  *                           row-end blocks: 4, 8 or 16
  *   prelim_blocks_per_sm    resident blocks per SM of that DP's persistent grid, 1..6

@@ -264,8 +264,9 @@ struct rmb_queries {
     std::mutex mu;
     DBuf d_qm, d_qmrc;   // DUST-masked queries and their reverse complements
     bool dusted = false;
-    DBuf d_dp;           // the packed-row DP's copies
+    DBuf d_dp, d_odd;    // the packed-row DP's copies and `odd`
     uint64_t dp_stride = 0;
+    uint32_t odd = 0;    // 32-base stretches with an ambiguity code other than N
     bool dp_made = false;
     void release() {
         d_q.release();
@@ -275,6 +276,7 @@ struct rmb_queries {
         d_qm.release();
         d_qmrc.release();
         d_dp.release();
+        d_odd.release();
     }
 };
 
@@ -406,11 +408,23 @@ void finish_query(const rmb_ctx& C, std::vector<Hit>& v, uint32_t qlen) {
     sort_hit_list_order(v, C.ids);
 }
 
+// Whether the packed-row DP takes a range's records (up to n_rec).  Its rows score the bases and N: a record
+// that meets another ambiguity code passes k_prelim_dual and k_prelim_pack and then takes a warp of its own.
+// So k_prelim_stream takes them all where that is many records and a large part of them, past one 32-base
+// stretch of the queries in 200 with such a code and 7,500 records that start in one.  Measured (B200,
+// preliminary DP ms, packed rows / k_prelim_stream): 40 queries of 60 kb against 500 consensi, 1.4 M records, no
+// such code 7.9 / 13.6, in 0.45 % of the stretches 13.8 / 13.7, 0.64 % 15.3 / 13.6, 3 % 26.7 / 13.7, 27 % 40.8 / 12.2;
+// one query of 60 kb against 2,000, 137,000 records, in 5 % 4.0 / 4.0; of 10 kb, 21,000 records, in 27 % 2.0 / 2.1;
+// of 1.5 kb, 1,700 records, in 88 % 0.54 / 1.23.
+bool pack_rows(const rmb_ctx& C, const DevQueries& Q, uint64_t n_rec) {
+    // the cell log covers the records that the thread-per-extension kernel completes
+    return C.prelim_pack && !C.sched_log && (Q.odd <= 1.0 / 200 || Q.odd * (double)n_rec <= 7500);
+}
+
 // The packed-row DP's part of a launch shape: its sequence copies and, where k_prelim_dual runs
 // first, the list of up to n records between the two kernels.
-void pack_config(rmb_ctx& C, Work& W, const DevQueries& Q, uint64_t n, StreamLaunch& cfg) {
-    // the cell log covers the records that the thread-per-extension kernel completes
-    cfg.pack = C.prelim_pack && !C.sched_log;
+void pack_config(rmb_ctx& C, Work& W, const DevQueries& Q, uint64_t n, bool pack, StreamLaunch& cfg) {
+    cfg.pack = pack;
     cfg.dual = cfg.pack && C.prelim_dual;
     if (cfg.pack) {
         W.pack_ctl.ensure(16);
@@ -464,6 +478,8 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     const bool bucket_fits = bucket_dedup_fits(npairs, nh);
     const bool leaders = fused && bucket_fits && nh >= (uint64_t)BUCKET_DENSE_HITS * npairs;
     const bool buckets = bucket_fits && (leaders || !fused);
+    // (where the hits a pair are many, the diagonal hash and the cutoff leave about one in 64)
+    const bool pack = pack_rows(C, Q, fused ? n1 / 64 : n1);
     if (!fused && !buckets) W.dd_scratch.ensure(dedup_threads(C.sms) * 1024 * 4);
     if (fused && !leaders) W.dd_units.ensure(dedup_units_bytes(npairs, nh, C.sms));
     W.ung_idx.ensure(n1 * 4);
@@ -501,7 +517,7 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     cfg.blocks_per_sm = tn.prelim_blocks_per_sm;
     cfg.window = tn.prelim_window;
     cfg.budget_div = tn.prelim_budget_div;
-    pack_config(C, W, Q, n1, cfg);
+    pack_config(C, W, Q, n1, pack, cfg);
     auto rec = [&](int k) { CK(cudaEventRecordWithFlags(W.ev[k], st, cudaEventRecordExternal)); };
 
     cudaGraph_t g = nullptr;
@@ -538,7 +554,7 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
         rec(1);
         const unsigned int* nu_dev = W.n_sel.as<unsigned int>();
         CK(launch_prelim_prep(C.L, Q, C.d_params.as<DevParams>(), n1, W.ung_idx.as<uint32_t>(), W.hits.as<SeedHit>(),
-                              W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms, st, C.prelim_pack, nu_dev));
+                              W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms, st, pack, nu_dev));
         const uint32_t* order = nullptr;
         rec(6);
         if (learned) {
@@ -729,8 +745,11 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
         if (C.prelim_pack && !QH.dp_made) {
             QH.dp_stride = dp_query_stride(QH.host.size(), nq);
             QH.d_dp.ensure(dp_bytes(4, QH.dp_stride));
+            QH.d_odd.ensure(4);
             CK(launch_dp_query(QH.d_q.as<uint8_t>(), QH.d_qrc.as<uint8_t>(), QH.d_off.as<uint64_t>(),
-                               QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride, st));
+                               QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride,
+                               QH.d_odd.as<unsigned int>(), st));
+            CK(cudaMemcpyAsync(&QH.odd, QH.d_odd.p, 4, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             QH.dp_made = true;
         }
@@ -798,7 +817,8 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
                      QH.d_off.as<uint64_t>() + qb, QH.d_len.as<uint32_t>() + qb, W.pv.as<uint32_t>(),
                      W.pv_off.as<uint64_t>(),    W.cs.as<uint32_t>(),     W.cs_off.as<uint64_t>(),
                      W.cq.as<uint32_t>(),        W.cq_off.as<uint64_t>(), C.lw.as<int32_t>() + qb, nb,
-                     QH.d_dp.as<uint8_t>(),      QH.dp_stride,            qb};
+                     QH.d_dp.as<uint8_t>(),      QH.dp_stride,            qb,
+                     (double)QH.odd * 32 / QH.host.size()};
         EvTimer ev;
         ev.start(st);
         {
@@ -1119,10 +1139,11 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
             EvTimer ev_main, es;  // es: the learned order's kernels
             bool es_used = false;
             if (C.prelim_stream) {
+                const bool pack = pack_rows(C, Q, nu);
                 W.geo.ensure(std::max<uint64_t>(nu, 1) * prelim_geo_bytes());
                 CK(launch_prelim_prep(C.L, Q, C.d_params.as<DevParams>(), nu, W.ung_idx.as<uint32_t>(),
                                       W.hits.as<SeedHit>(), W.hit_pair.as<uint32_t>(), W.ub.as<UngBox>(), W.geo.p, C.sms,
-                                      st, C.prelim_pack && !C.sched_log));
+                                      st, pack));
                 ctr.launches += nu ? 1 : 0;
                 const uint32_t* order = nullptr;
                 uint32_t* cells_out = nullptr;
@@ -1161,7 +1182,7 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
                 cfg.blocks_per_sm = tn.prelim_blocks_per_sm;
                 cfg.window = tn.prelim_window;
                 cfg.budget_div = tn.prelim_budget_div;
-                pack_config(C, W, Q, nu, cfg);
+                pack_config(C, W, Q, nu, pack, cfg);
                 CK(launch_prelim_stream(C.d_params.as<DevParams>(), nu, W.geo.p, W.po.as<PrelimOut>(),
                                         W.wide.as<uint32_t>(), W.n_wide.as<unsigned int>(),
                                         W.cells.as<unsigned long long>(), C.sms, st, order, cells_out,

@@ -51,6 +51,7 @@ struct DevQueries {
     const uint8_t* dp = nullptr;
     uint64_t dp_stride = 0;
     uint32_t q0 = 0;
+    double odd = 0;  // (host) the part of the set's 32-base stretches with an ambiguity code other than N
 };
 
 struct DevParams {

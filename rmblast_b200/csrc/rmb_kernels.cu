@@ -1707,20 +1707,29 @@ __global__ void __launch_bounds__(256) k_dp_nibbles(const uint2* __restrict__ in
     }
 }
 
-// Blocks (query, part of it); the bytes between the queries are filled by the caller.
+// Blocks (query, part of it); the bytes between the queries are filled by the caller.  *odd grows by the
+// number of 32-base stretches with a code 6, an ambiguity code other than N, in them.
 __global__ void __launch_bounds__(256) k_dp_query(const uint8_t* __restrict__ q, const uint8_t* __restrict__ qrc,
                                                   const uint64_t* __restrict__ off, const uint32_t* __restrict__ len,
-                                                  uint8_t* __restrict__ out, uint64_t stride) {
+                                                  uint8_t* __restrict__ out, uint64_t stride, unsigned int* __restrict__ odd) {
     const uint64_t o = off[blockIdx.x];
-    const uint32_t n = len[blockIdx.x];
+    const uint32_t n = len[blockIdx.x], lane = threadIdx.x & 31;
     uint8_t* d = out + o + (uint64_t)PACK_PAD * (blockIdx.x + 1);
-    for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.y * blockDim.x) {
-        const uint8_t f = (uint8_t)pack_sel(q[o + 1 + i] & 15u), r = (uint8_t)pack_sel(qrc[o + 1 + i] & 15u);
-        d[i] = f;
-        d[stride + n - 1 - i] = f;
-        d[2 * stride + i] = r;
-        d[3 * stride + n - 1 - i] = r;
+    unsigned int n_odd = 0;
+    for (uint64_t i0 = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x - lane; i0 < n; i0 += (uint64_t)gridDim.y * blockDim.x) {
+        const uint64_t i = i0 + lane;
+        uint8_t f = 0;
+        if (i < n) {
+            f = (uint8_t)pack_sel(q[o + 1 + i] & 15u);
+            const uint8_t r = (uint8_t)pack_sel(qrc[o + 1 + i] & 15u);
+            d[i] = f;
+            d[stride + n - 1 - i] = f;
+            d[2 * stride + i] = r;
+            d[3 * stride + n - 1 - i] = r;
+        }
+        n_odd += __any_sync(0xffffffffu, pack_odd(f) != 0);
     }
+    if (lane == 0 && n_odd) atomicAdd(odd, n_odd);
 }
 
 // The ring of a block: band entry j of thread x at ring[(j % STREAM_RING) * STREAM_BLOCK + x], so
@@ -2842,11 +2851,12 @@ cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const ui
 }
 
 cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t* off, const uint32_t* len, uint32_t nq,
-                            uint8_t* out, uint64_t stride, cudaStream_t st) {
+                            uint8_t* out, uint64_t stride, unsigned int* odd, cudaStream_t st) {
     if (!nq) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(out, PACK_BLOCKED, 4 * stride, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(odd, 0, sizeof *odd, st);
     if (e != cudaSuccess) return e;
-    k_dp_query<<<dim3(nq, query_parts(stride, nq)), 256, 0, st>>>(q, qrc, off, len, out, stride);
+    k_dp_query<<<dim3(nq, query_parts(stride, nq)), 256, 0, st>>>(q, qrc, off, len, out, stride, odd);
     return dp_pack(out, 4, stride, 0, st);
 }
 
