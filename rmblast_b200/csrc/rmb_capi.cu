@@ -2317,10 +2317,15 @@ int rmb_autotune(rmb_ctx* C, uint32_t nq, const uint8_t* const* query, const uin
                     }
                 }
             };
-            knob(&rmb_tune::prelim_group, {4, 16});
-            knob(&rmb_tune::prelim_blocks_per_sm, {4, 5});
+            // where the packed rows take every record of the sample, these three reach no launch, and a
+            // candidate could only win by noise
+            const bool stream = !C->prelim_pack || H->odd;
+            if (stream) {
+                knob(&rmb_tune::prelim_group, {4, 16});
+                knob(&rmb_tune::prelim_blocks_per_sm, {4, 5});
+            }
             knob(&rmb_tune::prelim_window, {32, 48});
-            knob(&rmb_tune::prelim_budget_div, {32, 512});
+            if (stream) knob(&rmb_tune::prelim_budget_div, {32, 512});
             knob(&rmb_tune::ungapped_blocks_per_sm, {4, 6});
             knob(&rmb_tune::dedup_extend_hits_per_pair, {0, -1});
             C->tune = cur;

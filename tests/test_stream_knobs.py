@@ -47,3 +47,18 @@ def test_knobs_leave_output_unchanged(name, scale, gaps):
 def test_plain_pipeline_matches_the_oracle(gaps):
     dbf, p, want, enc, ids = case(gaps, "plain", 0.005)
     assert searcher(p, synth.MATRIX_TEXT, synth.MATRIX_NAME, dbf, pipeline=1).search(enc, ids).tabular(FIELDS) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,scale", [("plain", 0.01), ("allvsall", 0.03)])
+def test_autotune_leaves_knobs_that_reach_no_launch(name, scale):
+    """Where the packed rows take every record, the thread-per-extension DP's knobs stay at their defaults."""
+    qf, dbf, p = synthetic(name, scale, synth.RM_FLAGS)
+    s = searcher(p, synth.MATRIX_TEXT, synth.MATRIX_NAME, dbf)
+    default = s.tune()
+    enc = [api.encode(x) for _, x in api.read_fasta(qf)]
+    for _ in range(3):
+        r = s.autotune(enc)
+        assert r["tune"] == s.tune() and r["best_ms"] <= r["default_ms"]
+        for k in ("prelim_group", "prelim_blocks_per_sm", "prelim_budget_div"):
+            assert s.tune()[k] == default[k], k
