@@ -1,7 +1,8 @@
 #pragma once
 // The ungapped X-drop extension of one word hit (search/ungapped.rs:38-121) as a resumable walk:
-// the left walk from the seed, then the right walk.  UngWalk is its plain form, one base a step, checked
-// on the host against the oracle's extension; UngBlocks the kernels' form, eight bases a step.
+// the left walk from the seed, then the right walk.  UngWalk is its plain form, one base a step; UngBlocks
+// the kernels' form, eight bases a step.  Both compile for the host too, where the tests check them against
+// the oracle's extension.
 #include <cstdint>
 
 namespace rmb {
@@ -79,14 +80,40 @@ struct UngWalk {
 };
 
 #ifdef __CUDACC__
-// The walks' score table in shared memory: entry ung_slot(a, c) for query code a, subject code c, so that
-// the 16 pairs of bases lie in 16 banks; a code 15 on either side (a sequence's end) ends any walk.
+__host__ __device__ __forceinline__ uint2 ung_load(const uint2* p) {
+#ifdef __CUDA_ARCH__
+    return __ldg(p);
+#else
+    return *p;
+#endif
+}
+__host__ __device__ __forceinline__ uint32_t ung_bytes(uint32_t lo, uint32_t hi, uint32_t sel) {  // __byte_perm
+#ifdef __CUDA_ARCH__
+    return __byte_perm(lo, hi, sel);
+#else
+    const uint64_t w = lo | (uint64_t)hi << 32;
+    uint32_t r = 0;
+    for (int k = 0; k < 4; ++k) r |= (uint32_t)(w >> 8 * (sel >> 4 * k & 7u) & 0xffu) << 8 * k;
+    return r;
+#endif
+}
+__host__ __device__ __forceinline__ uint32_t ung_shift(uint32_t lo, uint32_t hi, uint32_t by) {  // __funnelshift_r
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, by);
+#else
+    return (uint32_t)((lo | (uint64_t)hi << 32) >> (by & 31u));
+#endif
+}
+
+// The walks' score table: entry ung_slot(16 a + c) for query code a, subject code c, so that in shared
+// memory the 16 pairs of bases lie in 16 banks; a code 15 on either side (a sequence's end) ends any walk.
 constexpr int32_t UNG_END = -(1 << 30), UNG_XMAX = 1 << 29;  // (an X-drop past it is out of any walk's reach)
+__host__ __device__ __forceinline__ int ung_slot(int i) { return i ^ ((i >> 4 & 2) << 1); }
+__host__ __device__ __forceinline__ int32_t ung_entry(int i, const int32_t* matrix) {
+    return i >> 4 == 15 || (i & 15) == 15 ? UNG_END : matrix[i];
+}
 __device__ __forceinline__ void ung_table(int32_t* tab, const int32_t* __restrict__ matrix) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        const int a = i >> 4, c = i & 15;
-        tab[i ^ ((a & 2) << 1)] = a == 15 || c == 15 ? UNG_END : matrix[i];
-    }
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) tab[ung_slot(i)] = ung_entry(i, matrix);
 }
 
 // UngWalk eight bases a step.  A step's codes are two aligned words a sequence, one of them kept from
@@ -107,15 +134,15 @@ struct UngBlocks {
     int32_t x, xc, sum, score, n, best, q_beg;  // n: bases walked; best: of them, up to the best sum
     bool left;
 
-    __device__ __forceinline__ uint2 word(const uint2* p) const {
-        const uint2 w = __ldg(p);
+    __host__ __device__ __forceinline__ uint2 word(const uint2* p) const {
+        const uint2 w = ung_load(p);
         const uint32_t s0 = left ? 0x4567u : 0x3210u, s1 = left ? 0x0123u : 0x7654u;
-        return make_uint2(__byte_perm(w.x, w.y, s0), __byte_perm(w.x, w.y, s1));
+        return make_uint2(ung_bytes(w.x, w.y, s0), ung_bytes(w.x, w.y, s1));
     }
-    __device__ __forceinline__ const uint2* after(const Side& s) const {  // stays at the walk's end
+    __host__ __device__ __forceinline__ const uint2* after(const Side& s) const {  // stays at the walk's end
         return s.at == s.last ? s.at : left ? s.at - 1 : s.at + 1;
     }
-    __device__ __forceinline__ void enter(Side& s, const uint8_t* seq, int32_t len, int32_t i) {
+    __host__ __device__ __forceinline__ void enter(Side& s, const uint8_t* seq, int32_t len, int32_t i) {
         const uint64_t p = (uint64_t)(seq + 1 + i);
         s.last = (const uint2*)((uint64_t)(left ? seq : seq + 1 + len) & ~7ull);
         s.at = (const uint2*)(p & ~7ull);
@@ -125,17 +152,17 @@ struct UngBlocks {
         s.next = word(s.at);
         s.at = after(s);
     }
-    __device__ __forceinline__ uint2 codes(Side& s) {
+    __host__ __device__ __forceinline__ uint2 codes(Side& s) {
         const bool high = s.shift >= 32;
         const uint32_t w0 = high ? s.cur.y : s.cur.x, w1 = high ? s.next.x : s.cur.y, w2 = high ? s.next.y : s.next.x;
         s.cur = s.next;
         s.next = word(s.at);
         s.at = after(s);
-        return make_uint2(__funnelshift_r(w0, w1, s.shift & 31u), __funnelshift_r(w1, w2, s.shift & 31u));
+        return make_uint2(ung_shift(w0, w1, s.shift & 31u), ung_shift(w1, w2, s.shift & 31u));
     }
     // From the seed (wq, wsx) with X-drop xdrop: the left walk first.
-    __device__ __forceinline__ void start(const uint8_t* query, const uint8_t* subject, int32_t query_len,
-                                          int32_t subject_len, int32_t seed_q, int32_t seed_s, int32_t xdrop) {
+    __host__ __device__ __forceinline__ void start(const uint8_t* query, const uint8_t* subject, int32_t query_len,
+                                                   int32_t subject_len, int32_t seed_q, int32_t seed_s, int32_t xdrop) {
         qb = query;
         sb = subject;
         qlen = query_len;
@@ -149,7 +176,7 @@ struct UngBlocks {
         enter(c, sb, slen, wsx - 1);
     }
     // Up to eight bases; true when the right walk has ended.
-    __device__ __forceinline__ bool step(const int32_t* tab) {
+    __host__ __device__ __forceinline__ bool step(const int32_t* tab) {
         const uint2 qa = codes(a), sc = codes(c);
         bool run = true;
 #pragma unroll
@@ -181,7 +208,8 @@ struct UngBlocks {
         return false;
     }
     // After step() returned true: the extension in the walk's frame.
-    __device__ __forceinline__ void result(int32_t& sc, uint32_t& q0, uint32_t& q1, uint32_t& s0, uint32_t& s1) const {
+    __host__ __device__ __forceinline__ void result(int32_t& sc, uint32_t& q0, uint32_t& q1, uint32_t& s0,
+                                                    uint32_t& s1) const {
         sc = score;
         q0 = (uint32_t)q_beg;
         q1 = (uint32_t)(wq + best);
