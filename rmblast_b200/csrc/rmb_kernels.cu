@@ -2738,11 +2738,11 @@ bool prelim_stream_eligible(const int32_t* matrix256, int32_t gap_open, int32_t 
 // decays a signed byte, and a blocked column's score of -128 has to end every path.
 bool prelim_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop_gap) {
     const int32_t goe = gap_open + gap_extend, xmax = std::max(xdrop_gap, goe);
-    if (gap_extend < 1 || gap_open < 0 || xmax > PACK_XMAX) return false;
+    if (gap_extend < 1 || gap_extend > PACK_GE_MAX || gap_open < 0 || xmax > PACK_XMAX) return false;
     if ((xmax - goe) / gap_extend + 1 > 16) return false;
     for (int a = 0; a < 16; ++a)
         for (int b : {0, 1, 2, 3, 14})
-            if (matrix256[a * 16 + b] + 2 * gap_extend > 127) return false;
+            if (matrix256[a * 16 + b] + 2 * gap_extend > PACK_STEP_MAX) return false;
     return true;
 }
 
@@ -3028,7 +3028,7 @@ bool traceback_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t
     // the initial row right of the pivot's diagonal, and 16-bit values: best + origin up to PACK_REBASE
     // and a row's gain, the diagonals' decay over the window on top
     const int32_t goe = gap_open + gap_extend, xmax = std::max(xdrop, goe);
-    if (gap_extend < 1 || gap_extend > 40 || gap_open < 0 || xmax > 4000) return false;
+    if (gap_extend < 1 || gap_extend > TB_GE_MAX || gap_open < 0 || xmax > TB_XMAX) return false;
     if ((xmax - goe) / gap_extend + 1 + TB_K >= TB_W - 1) return false;
     // a dead cell is 0 and the lowest live value, one X below a best of 0 in the first row, TB_LIVE + 2 gap_extend
     // on the first window diagonal: a score with its decay has to stay below it

@@ -44,9 +44,15 @@
 namespace rmb {
 
 constexpr int DUAL_W = 56, DUAL_K = 26, DUAL_ROWS = 8, DUAL_SHIFT = 4, DUAL_BLOCK = 128;
-// best + origin may pass DUAL_REBASE by a batch, a window move and a record's start (under 1,100) and a
-// cell lies 63 * 55 above at most: below 0x7c00; what is left after the move keeps live values above 255
+// Between two looks best + origin grows past DUAL_REBASE by a window move, a record's start (PACK_STEP_MAX + 1
+// and its X) and a batch's rows, 1,524 at most; a cell's diagonal lies up to 63 * 55 above: together below
+// 0x7c00, where half floats stop ordering as integers.  What is left after the origin's move keeps the
+// threshold above what a dead cell can reach in a row.
 constexpr int32_t DUAL_REBASE = 24576, DUAL_REBASE_BY = 24064;
+static_assert(DUAL_REBASE + DUAL_SHIFT * PACK_GE_MAX + PACK_STEP_MAX + 1 + PACK_XMAX + DUAL_ROWS * PACK_STEP_MAX +
+                      (DUAL_W - 1) * PACK_GE_MAX < 0x7c00, "the values stay finite half floats");
+static_assert(DUAL_REBASE - DUAL_REBASE_BY - PACK_XMAX > PACK_STEP_MAX, "a dead cell stays dead after the origin's move");
+static_assert(DUAL_SHIFT <= 2 * DUAL_ROWS, "moves to the left lower the origin by less than the rows raise it");
 constexpr int DUAL_BITS = 10;  // columns of a half-precision bit mask
 constexpr int DUAL_MASKS = (DUAL_W + DUAL_BITS - 1) / DUAL_BITS;
 
@@ -153,8 +159,8 @@ k_prelim_dual(const DevParams* __restrict__ P, const __grid_constant__ DualConst
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 DualCold& k = cold[h][threadIdx.x];
-                // a first step adds 127 at most to what the half still holds, all of it at most its best
-                const int32_t top = (int32_t)(h ? pb >> 16 : pb & 0xffffu) + 128;
+                // a first step adds PACK_STEP_MAX at most to what the half still holds, all of it at most its best
+                const int32_t top = (int32_t)(h ? pb >> 16 : pb & 0xffffu) + PACK_STEP_MAX + 1;
                 while ((ended >> h & 1u) && phase[h] != 4) {
                     const int32_t best = (int32_t)((h ? pb >> 16 : pb & 0xffffu)) - org[h];
                     if (phase[h] != 0) {

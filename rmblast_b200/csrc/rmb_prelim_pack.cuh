@@ -32,6 +32,8 @@ namespace rmb {
 
 constexpr int PACK_BLOCK = 128;
 constexpr int PACK_XMAX = 128;        // a blocked column's score is -128: it has to end any path
+constexpr int PACK_STEP_MAX = 127;    // a score with both gaps' decay, 2 gap_extend, in a signed byte
+constexpr int PACK_GE_MAX = 63;       // the largest gap_extend that leaves a positive score under it
 constexpr int32_t PACK_REBASE = 16384, PACK_REBASE_BY = 8192;
 
 // The launch's constants: packed pairs (the same value in both halves), by register
@@ -100,6 +102,8 @@ k_prelim_pack(const DevParams* __restrict__ P, const __grid_constant__ PackConst
     constexpr int W = 2 * G * R;
     constexpr int K_OFF = W / 2 - 2;  // the window diagonal of the pivot's diagonal at the start
     static_assert(2 * R <= 16 && K_OFF + 17 < W - 1, "a lane's residues are four words; the widest initial row fits");
+    static_assert(PACK_REBASE + PACK_STEP_MAX + R * PACK_GE_MAX + (W - 1) * PACK_GE_MAX < 0x8000, "the values fit 16 bits");
+    static_assert(PACK_REBASE - PACK_REBASE_BY - PACK_XMAX > PACK_STEP_MAX, "a dead cell stays dead after the origin's move");
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ uint2 tab[16];
     const int32_t ge = P->gap_extend, go = P->gap_open, goe = go + ge;

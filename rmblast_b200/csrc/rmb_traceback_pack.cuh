@@ -24,6 +24,10 @@ constexpr int TB_R = 2, TB_W = 64 * TB_R, TB_K = TB_W / 2 - 2;
 constexpr uint32_t TB_ROW_BYTES = TB_W / 2 + 4;  // trace and window position of a row
 constexpr int32_t TB_SCORE_MIN = -8192;          // a blocked column's score: ends any path
 constexpr int32_t TB_LIVE = 256;                 // live values stay above it: no score of a cell reaches it
+constexpr int32_t TB_GE_MAX = 40, TB_XMAX = 4000;
+static_assert(PACK_REBASE + TB_LIVE + (2 + 2 * TB_R) * TB_GE_MAX + (TB_W - 1) * TB_GE_MAX < 0x8000, "the values fit 16 bits");
+static_assert(PACK_REBASE - PACK_REBASE_BY - TB_XMAX > TB_LIVE + 2 * TB_GE_MAX, "a dead cell stays dead after the origin's move");
+static_assert(-TB_SCORE_MIN > TB_XMAX + 2 * TB_GE_MAX, "a blocked column ends any path");
 
 // Status of an extension that its window or its codes do not fit: the byte-trace kernel takes it.
 constexpr int TB_WIDE = 4;
