@@ -2357,6 +2357,7 @@ __global__ void __launch_bounds__(128) k_traceback_pack(DevLib L, DevQueries Q, 
         }
         tab.row[threadIdx.x] = make_uint4(lo[0], lo[1], hi[0], hi[1]);
     }
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) tab.all[i] = (int16_t)max(P->matrix[i] + 2 * ge, TB_SCORE_MIN);
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

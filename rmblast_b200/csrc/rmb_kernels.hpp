@@ -157,7 +157,7 @@ cudaError_t launch_prelim_wide(const DevLib& L, const DevQueries& Q, const DevPa
                                const UngBox* ub, PrelimOut* out, int2* band_mem, uint64_t band_cap, uint32_t threads,
                                unsigned long long* cells, unsigned int* failures, cudaStream_t st, const unsigned int* n_dev = nullptr);
 // The traceback with the band in registers: `warps` (a multiple of 4) slots of traceback_pack_bytes(rows_cap)
-// in scratch.  Status 4 (the window or the codes did not fit) takes launch_traceback.
+// in scratch.  Status 4 (the window did not fit) takes launch_traceback.
 bool traceback_pack_eligible(const int32_t* matrix256, int32_t gap_open, int32_t gap_extend, int32_t xdrop);
 uint64_t traceback_pack_bytes(uint32_t rows_cap);
 cudaError_t launch_traceback_pack(const DevLib& L, const DevQueries& Q, const DevParams* P, uint32_t n, const TbIn* in,

@@ -5,7 +5,8 @@
 // The rows are k_prelim_pack's (rmb_prelim_pack.cuh: window of diagonals, packed 16-bit values,
 // coordinates, exactness), with the whole warp on one extension, TB_W = 128 diagonals, four a lane.  The
 // scores are 16-bit table entries (two byte lookups and a merge), so the X-drop is limited by the
-// window alone, and the scores by what keeps a dead cell dead (TB_LIVE).  A cell's trace is four bits:
+// window alone, and the scores by what keeps a dead cell dead (TB_LIVE).  They hold the bases and N; a
+// column of another ambiguity code looks its score up in shared memory.  A cell's trace is four bits:
 // the vertical gap beat the diagonal, the horizontal gap beat both, and either gap's extension is at
 // least its opening, gapped.rs:577-618's op byte; a row's 128 are 64 bytes, one 16-bit store a lane,
 // with the row's window position beside them.  On cells below the X-drop threshold they may differ
@@ -29,11 +30,12 @@ static_assert(PACK_REBASE + TB_LIVE + (2 + 2 * TB_R) * TB_GE_MAX + (TB_W - 1) * 
 static_assert(PACK_REBASE - PACK_REBASE_BY - TB_XMAX > TB_LIVE + 2 * TB_GE_MAX, "a dead cell stays dead after the origin's move");
 static_assert(-TB_SCORE_MIN > TB_XMAX + 2 * TB_GE_MAX, "a blocked column ends any path");
 
-// Status of an extension that its window or its codes do not fit: the byte-trace kernel takes it.
+// Status of an extension that its window does not fit: the byte-trace kernel takes it.
 constexpr int TB_WIDE = 4;
 
 struct TbTable {  // scores with both gap decays: row residue x code, low and high bytes of codes 0-3, 4-7
     uint4 row[16];
+    int16_t all[256];  // the same for every pair of residues
 };
 
 __device__ __forceinline__ uint32_t tb_code(uint32_t base) { return base < 4 ? base : base == 14 ? 4u : 6u; }
@@ -81,7 +83,7 @@ __device__ __forceinline__ int tb_pack_extend(const uint8_t* __restrict__ a, con
             S[r] = 0;
         }
     }
-    if (__any_sync(FULL, odd)) return TB_WIDE;
+    bool codes = __any_sync(FULL, odd);  // some column of the window has code 6
     uint32_t pb = pack2(bo, bo) + half_base;
     uint32_t a_cur = a[0] & 15u, a_nx = m > 1 ? a[dir] & 15u : 0u;
     uint32_t b_nx = code_at(W - TB_K);  // the last diagonal's code in the second row
@@ -93,11 +95,31 @@ __device__ __forceinline__ int tb_pack_extend(const uint8_t* __restrict__ a, con
         uint32_t x = __shfl_down_sync(FULL, E[0], 1);
         if (lane == 31) x = 0;
         const uint32_t e_edge = prmt(E[0], x, 0x5432);
-        uint32_t f = 0, p = pb, D[R], T[R], F[R], pr[R];
+        uint32_t f = 0, p = pb, D[R], T[R], F[R], pr[R], sc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) sc[r] = prmt(prmt(tb.x, tb.y, sel[r]), prmt(tb.z, tb.w, sel[r]), 0x6240);
+        // Code 6, an ambiguity code other than N: the residue's own score, while the window has one.  (Such
+        // extensions went to k_traceback_warp before: 40 queries of 60 kb against 500 consensi with 0.05 % of such
+        // codes 28.5 ms, 9.2 now, with 1 % 28.6 and 12.9.)
+        if (codes) {
+            bool some = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int32_t j = col0 + r + k0 + row;
+                if ((sel[r] & 0xffu) == 6) {
+                    sc[r] = (sc[r] & 0xffff0000u) | (uint16_t)tab.all[a_cur * 16 + (b[(ptrdiff_t)dir * j] & 15u)];
+                    some = true;
+                }
+                if ((sel[r] >> 8 & 0xffu) == 6) {
+                    sc[r] = (sc[r] & 0xffffu) | (uint32_t)(uint16_t)tab.all[a_cur * 16 + (b[(ptrdiff_t)dir * (j + R)] & 15u)] << 16;
+                    some = true;
+                }
+            }
+            codes = __any_sync(FULL, some);
+        }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const uint32_t sc = prmt(prmt(tb.x, tb.y, sel[r]), prmt(tb.z, tb.w, sel[r]), 0x6240);
-            D[r] = __viaddmax_s16x2_relu(H[r], sc, 0u);
+            D[r] = __viaddmax_s16x2_relu(H[r], sc[r], 0u);
             T[r] = __vmaxs2(D[r], r + 1 < R ? E[r + 1 < R ? r + 1 : r] : e_edge);
             F[r] = f;
             f = __viaddmax_s16x2(T[r], neg_go, f);
@@ -166,7 +188,7 @@ __device__ __forceinline__ int tb_pack_extend(const uint8_t* __restrict__ a, con
             const uint32_t s0 = sel[0];
             uint32_t sn = __shfl_down_sync(FULL, s0, 1);
             if (lane == 31) sn = b_nx;
-            if (__any_sync(FULL, lane == 31 && b_nx == 6)) return TB_WIDE;
+            codes |= __any_sync(FULL, lane == 31 && b_nx == 6) != 0;
 #pragma unroll
             for (int r = 0; r + 1 < R; ++r) sel[r] = sel[r + 1];
             sel[R - 1] = prmt(s0, sn, 0x0041);
@@ -200,7 +222,8 @@ __device__ __forceinline__ int tb_pack_extend(const uint8_t* __restrict__ a, con
             bo += ge * by;
             pb += (uint32_t)(ge * by) * 0x00010001u;
             if (lane == 31) b_nx = code_at(W + k0 + row);
-            if (__any_sync(FULL, odd)) return TB_WIDE;
+            codes |= __any_sync(FULL, odd) != 0;
+            odd = false;
         }
         if (bo > PACK_REBASE) {
             const uint32_t by = pack2(-PACK_REBASE_BY, -PACK_REBASE_BY);
