@@ -264,7 +264,9 @@ struct rmb_queries {
     std::mutex mu;
     DBuf d_qm, d_qmrc;   // DUST-masked queries and their reverse complements
     bool dusted = false;
-    DBuf d_dp, d_odd;    // the packed-row DP's copies and `odd`
+    DBuf d_dp;           // the packed-row DP's copies
+    DBuf d_odd;          // launch_dp_query's count, and where the host reads it
+    HostBuf h_odd;
     uint64_t dp_stride = 0;
     uint32_t odd = 0;    // 32-base stretches with an ambiguity code other than N
     bool dp_made = false;
@@ -745,12 +747,16 @@ void run_core(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_hi
         if (C.prelim_pack && !QH.dp_made) {
             QH.dp_stride = dp_query_stride(QH.host.size(), nq);
             QH.d_dp.ensure(dp_bytes(4, QH.dp_stride));
-            QH.d_odd.ensure(4);
+            if (!QH.d_odd.p) {
+                QH.d_odd.ensure(4);
+                CK(cudaMemsetAsync(QH.d_odd.p, 0, 4, st));
+                QH.h_odd.resize(4);
+            }
             CK(launch_dp_query(QH.d_q.as<uint8_t>(), QH.d_qrc.as<uint8_t>(), QH.d_off.as<uint64_t>(),
                                QH.d_len.as<uint32_t>(), nq, QH.d_dp.as<uint8_t>(), QH.dp_stride,
-                               QH.d_odd.as<unsigned int>(), st));
-            CK(cudaMemcpyAsync(&QH.odd, QH.d_odd.p, 4, cudaMemcpyDeviceToHost, st));
+                               QH.d_odd.as<unsigned int>(), (unsigned int*)QH.h_odd.data(), st));
             CK(cudaStreamSynchronize(st));
+            memcpy(&QH.odd, QH.h_odd.data(), 4);
             QH.dp_made = true;
         }
     }

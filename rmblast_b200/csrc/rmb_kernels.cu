@@ -1694,9 +1694,15 @@ __global__ void __launch_bounds__(256) k_dp_subject(const uint8_t* __restrict__ 
     }
 }
 
-// The codes of a byte copy, eight to a word: bits sh .. sh + 3 of each byte.
+// The codes of a byte copy, eight to a word: bits sh .. sh + 3 of each byte.  k_dp_query's count goes to the
+// host's word, and its own starts again at zero (a memset and a copy took 12 us of a short search).
 __global__ void __launch_bounds__(256) k_dp_nibbles(const uint2* __restrict__ in, uint64_t n_words, int sh,
-                                                    uint32_t* __restrict__ out) {
+                                                    uint32_t* __restrict__ out, unsigned int* __restrict__ odd,
+                                                    unsigned int* __restrict__ odd_host) {
+    if (odd && blockIdx.x == 0 && threadIdx.x == 0) {
+        *odd_host = *odd;
+        *odd = 0;
+    }
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words; w += (uint64_t)gridDim.x * blockDim.x) {
         uint2 v = in[w];
         v.x = (v.x >> sh) & 0x0f0f0f0fu;
@@ -2835,10 +2841,11 @@ cudaError_t launch_prelim_prep(const DevLib& L, const DevQueries& Q, const DevPa
     return cudaGetLastError();
 }
 
-static cudaError_t dp_pack(uint8_t* dp, int copies, uint64_t stride, int sh, cudaStream_t st) {
+static cudaError_t dp_pack(uint8_t* dp, int copies, uint64_t stride, int sh, unsigned int* odd, unsigned int* odd_host,
+                           cudaStream_t st) {
     const uint64_t n = copies * stride / 8;
     k_dp_nibbles<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 8192), 256, 0, st>>>(
-        (const uint2*)dp, n, sh, const_cast<uint32_t*>(dp_nibbles(dp, copies, stride)));
+        (const uint2*)dp, n, sh, const_cast<uint32_t*>(dp_nibbles(dp, copies, stride)), odd, odd_host);
     return cudaGetLastError();
 }
 
@@ -2848,17 +2855,16 @@ cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const ui
     cudaError_t e = cudaMemsetAsync(out, 15 * 8, 2 * stride, st);
     if (e != cudaSuccess) return e;
     k_dp_subject<<<n, 256, 0, st>>>(plus, off, len, out, stride);
-    return dp_pack(out, 2, stride, 3, st);
+    return dp_pack(out, 2, stride, 3, nullptr, nullptr, st);
 }
 
 cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t* off, const uint32_t* len, uint32_t nq,
-                            uint8_t* out, uint64_t stride, unsigned int* odd, cudaStream_t st) {
+                            uint8_t* out, uint64_t stride, unsigned int* odd, unsigned int* odd_host, cudaStream_t st) {
     if (!nq) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(out, PACK_BLOCKED, 4 * stride, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(odd, 0, sizeof *odd, st);
     if (e != cudaSuccess) return e;
     k_dp_query<<<dim3(nq, query_parts(stride, nq)), 256, 0, st>>>(q, qrc, off, len, out, stride, odd);
-    return dp_pack(out, 4, stride, 0, st);
+    return dp_pack(out, 4, stride, 0, odd, odd_host, st);
 }
 
 cudaError_t launch_prelim_stream(const DevParams* P, uint64_t n, const void* geo, PrelimOut* out, uint32_t* wide,

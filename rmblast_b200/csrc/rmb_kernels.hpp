@@ -119,9 +119,10 @@ uint64_t dp_subject_stride(uint64_t bytes, uint32_t n);
 cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const uint32_t* len, uint32_t n, uint8_t* out,
                               uint64_t stride, cudaStream_t st);
 uint64_t dp_query_stride(uint64_t bytes, uint32_t nq);
-// (*odd: the 32-base stretches of the queries that hold an ambiguity code other than N)
+// (*odd_host, pinned: the 32-base stretches of the queries that hold an ambiguity code other than N, counted
+// in *odd, zero before and after)
 cudaError_t launch_dp_query(const uint8_t* q, const uint8_t* qrc, const uint64_t* off, const uint32_t* len, uint32_t nq,
-                            uint8_t* out, uint64_t stride, unsigned int* odd, cudaStream_t st);
+                            uint8_t* out, uint64_t stride, unsigned int* odd, unsigned int* odd_host, cudaStream_t st);
 cudaError_t launch_prelim_stream(const DevParams* P, uint64_t n, const void* geo, PrelimOut* out, uint32_t* wide,
                                  unsigned int* n_wide, unsigned long long* cells, int sms, cudaStream_t st,
                                  const uint32_t* order, uint32_t* cells_out, bool plain, const StreamLaunch& cfg,
