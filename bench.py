@@ -41,12 +41,12 @@ sys.path.insert(0, str(ROOT))
 
 FIELDS = "6 score perc_sub qseqid qstart qend sseqid sstart send"
 OPS_PER_CELL = 11  # int32 add/sub/max/compare per DP cell in search/gapped.rs:234-262
-# DRAM bytes (read + write) per ungapped record of the preliminary DP, from one ncu capture of the
-# kernel's int32 form on `bench.py --workload plain --scale 0.01` (1.31 M records, 80.1 MB); the
-# traffic is per record (the 48-byte geometry read, the 28-byte result write, sequence words), the
-# same in the packed form, so a launch's traffic is this times its records
-PRELIM_DRAM_BYTES_PER_RECORD = 61.0
-# copy bandwidth of this pool's B200s measured earlier, used when MEASURED_PEAKS.json is absent
+# DRAM bytes (read + write) per ungapped record of the preliminary DP, from one ncu capture of k_prelim_dual,
+# k_prelim_pack and k_prelim_pack_join: 60 queries of 60 kb against 1,000 consensi, 4.13 M records, 328 MB
+# (the 48-byte geometry read, the 28-byte result written, sequence words); a launch's traffic is this
+# times its records
+PRELIM_DRAM_BYTES_PER_RECORD = 79.0
+# copy bandwidth of a B200 measured earlier, used when MEASURED_PEAKS.json is absent
 HBM_FALLBACK_GBS = 6650.0
 BATCH_CHUNKS = 1000
 
@@ -454,9 +454,10 @@ def main():
                              "frac": (traffic / (main_ms * 1e-3) / 1e9 / peaks["hbm_gbs"]
                                       if traffic and peaks.get("hbm_gbs") else None)},
                      "note": f"{OPS_PER_CELL} int32 ops per DP cell (the reference's cell step) x cells of the "
-                             "records these kernels completed / their event time (they take two cells an "
-                             "operation, in 16-bit halves); peak = rmb_probe_int32_peak "
-                             "(dependent int32 add/max throughput of this GPU) measured in this run; the kernels "
+                             "records these kernels completed / their event time; peak = rmb_probe_int32_peak "
+                             "(dependent int32 add/max throughput of this GPU) measured in this run; the kernels take "
+                             "two cells an operation, in 16-bit halves, on a pipe of half that rate, so the peak is "
+                             "the same number, and some of the 11 operations on the multiply-add pipe beside it; they "
                              "are bound by integer issue, not by HBM (hbm.frac) or tensor cores"},
         "gpu_launches": int(c["launches"] * args.steps),
         "clocks": clk,

@@ -474,9 +474,10 @@ void chain_graph(rmb_ctx& C, Work& W, const DevQueries& Q, int32_t ucut, uint64_
     const rmb_tune& tn = C.tune;
     // The bucket replay, of all hits extended first or, in dense ranges, of the leaders.  k_dedup_extend
     // keeps the dense ranges whose pairs hold few thousand hits: it extends no dropped hit, and a warp a
-    // pair is enough lanes there (40 consensi of 5 kb against their 1,000, 3,500 hits a pair: 20 ms to
-    // 34); over 8,192 hits a pair its rounds wait on one pair's buckets (100 kb against 50 consensi,
-    // 31,000 hits a pair: 10.6 ms to 0.7; 2.1 Mb against 50: 129 to 14).
+    // pair is enough lanes there; in longer lists its rounds wait on one pair's buckets.  Measured (B200,
+    // ms, k_dedup_extend / leaders) on consensi against each other, where the line lies: 1,400 hits a pair
+    // 0.77 / 1.24, 3,500 20 / 34, 9,900 5.9 / 4.9, 22,000 13.6 / 8.9, 61,000 39 / 21; on a genome against a library
+    // the leaders win earlier: 2,800 2.2 / 0.13, 10,700 3.4 / 0.33, 110,000 51 / 10.
     const bool bucket_fits = bucket_dedup_fits(npairs, nh);
     const bool leaders = fused && bucket_fits && nh >= (uint64_t)BUCKET_DENSE_HITS * npairs;
     const bool buckets = bucket_fits && (leaders || !fused);

@@ -61,9 +61,10 @@ struct PairView {
 // masked query; returns false if the word hit is dropped.  The two runs of matching bases beside the
 // word, at most ext_needed long, are counted in two loops of the whole warp (the sentinels at the
 // sequences' ends stop them; a loop ends when no lane's run goes on), then limited in the strand's
-// order: left first on the plus strand, right first on the minus strand.  Early returns out of the
-// loops are avoided on purpose: with them the warp was seen to reach the caller's vote in two parts
-// (one hit in millions lost).
+// order: left first on the plus strand, right first on the minus strand.  The whole warp runs it for
+// every candidate, without early returns.  A form that returned out of the loops gave the caller's vote 23
+// hits fewer of 93.7 M; why was not found.  This one's counts, pair by pair, are those of one position a
+// lane and round on all 2 M pairs of that search.
 __device__ __forceinline__ bool exact_extend(const PairView& v, bool there, uint32_t q0c, uint32_t p, uint32_t& qs,
                                              uint32_t& so) {
     const int64_t c1 = v.qlen + 1;
@@ -129,8 +130,8 @@ __device__ __forceinline__ uint64_t scan_unit_of(const ScanUnits& U, uint32_t n_
 // query bytes).  So a round takes SCAN_POS positions a lane, their loads side by side, and its cells'
 // entries are spread over the warp as one list, one entry a lane.  Measured (B200) against one position a
 // lane and round: 1,000 contigs against 2,000 consensi (2 M pairs) 31 -> 14.7 ms, 120 chunks of 60 kb
-// 8.2 -> 2.8, 4,000 sequences at word 14 11.3 -> 6.0; and by stretches of pairs, 100 kb at word 7
-// 5.5 -> 0.1, 2.1 Mb against 2,000 consensi 50 -> 1.
+// 8.2 -> 2.8, 4,000 sequences at word 14 11.3 -> 6.0; and by stretches of pairs (scan_segments), 100 kb
+// against 50 consensi at word 7 5.5 -> 0.09, 2.1 Mb (three chunks) 52 -> 0.97.
 enum { SCAN_WRITE = 1, SCAN_STAGE = 2 };
 constexpr int SCAN_POS = 4;
 constexpr uint32_t SCAN_ROUND = 32 * SCAN_POS;
@@ -2525,8 +2526,9 @@ std::vector<uint32_t> scan_segments(uint32_t n_queries, const std::vector<uint32
                                     double hits_per_position, int sms) {
     // A pair is one warp's while the pairs fill the chip's warp slots twice.  With fewer, a stretch is as
     // many rounds of the subject as spread the rounds over the slots, and no more than stage a quarter of
-    // SCAN_STAGE_PER_WARP (100 kb at word 7 against 50 consensi: a warp a pair took 5.5 ms, stretches
-    // 0.3; 2.1 Mb, 1.5 M hits in a pair: 50 ms with the pairs' stages overrun, 29 with 14 stretches each).
+    // SCAN_STAGE_PER_WARP.  Measured (B200), a warp a pair and stretches: 100 kb against 50 consensi at word 7
+    // 5.5 -> 0.09 ms; 2.1 Mb, three chunks, 0.9 M hits a pair, whose pairs overran their stages, 52 -> 0.97;
+    // 1.9 Mb in one chunk, where the busiest stretches still do, 89 -> 48; 2.1 Mb against 2,000 at word 11 0.73 -> 0.18.
     const uint64_t slots = (uint64_t)sms * 128, pairs = (uint64_t)n_queries * slen.size();
     if (!pairs || pairs >= slots) return {};
     uint64_t rounds = 0;
