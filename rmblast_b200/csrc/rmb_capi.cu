@@ -1812,10 +1812,13 @@ int rmb_db_load(rmb_ctx* C, uint32_t n, const uint8_t* const* plus, const uint32
         upload(C->d_plus_off, C->plus_off, st);
         upload(C->d_packed_off, C->packed_off, st);
         upload(C->d_len, C->slen, st);
-        const uint64_t dp_stride = dp_subject_stride(hplus.size(), n);
-        C->d_dp.ensure(dp_bytes(2, dp_stride));
-        CK(launch_dp_subject(C->d_plus.as<uint8_t>(), C->d_plus_off.as<uint64_t>(), C->d_len.as<uint32_t>(), n,
-                             C->d_dp.as<uint8_t>(), dp_stride, st));
+        uint64_t dp_stride = 0;
+        if (C->prelim_pack) {
+            dp_stride = dp_subject_stride(hplus.size(), n);
+            C->d_dp.ensure(dp_bytes(2, dp_stride));
+            CK(launch_dp_subject(C->d_plus.as<uint8_t>(), C->d_plus_off.as<uint64_t>(), C->d_len.as<uint32_t>(), n,
+                                 C->d_dp.as<uint8_t>(), dp_stride, st));
+        }
         CK(cudaStreamSynchronize(st));
         C->L = DevLib{C->d_plus.as<uint8_t>(),      C->d_rc.as<uint8_t>(),         C->d_align.as<uint8_t>(),
                       C->d_align_rc.as<uint8_t>(),  C->d_packed.as<uint8_t>(),     C->d_plus_off.as<uint64_t>(),
