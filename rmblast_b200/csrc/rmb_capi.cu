@@ -1735,7 +1735,8 @@ int rmb_ctx_create(const rmb_params* params, const int32_t scores[256], const do
         }
         if (p.evalue < 0.0) throw Fail(RMB_EINVAL, "evalue must be >= 0");
         C->d_params.ensure(sizeof(DevParams));
-        CK(cudaMemcpy(C->d_params.p, &dp, sizeof dp, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(C->d_params.p, &dp, sizeof dp, cudaMemcpyHostToDevice, C->st));
+        CK(cudaStreamSynchronize(C->st));
         *out = C;
         return RMB_OK;
     } catch (const Fail& e) {
@@ -2070,7 +2071,8 @@ void run_search(rmb_ctx& C, rmb_queries& QH, std::vector<std::vector<Hit>>& out_
         for (size_t k = 0; k < cmask.size(); ++k) memcpy(hm.data() + CH->off[k], cmask[k].data(), cmask[k].size());
         CH->d_qm.ensure(hm.size());
         CH->d_qmrc.ensure(hm.size());
-        CK(cudaMemcpy(CH->d_qm.p, hm.data(), hm.size(), cudaMemcpyHostToDevice));
+        // (on the stream that reads it: a copy on another one may still be under way when it returns)
+        CK(cudaMemcpyAsync(CH->d_qm.p, hm.data(), hm.size(), cudaMemcpyHostToDevice, C.st));
         CK(launch_revcomp(CH->d_qm.as<uint8_t>(), CH->d_off.as<uint64_t>(), CH->d_len.as<uint32_t>(), CH->n, CH->host.size(),
                           CH->d_qmrc.as<uint8_t>(), C.st));
         CK(cudaStreamSynchronize(C.st));
@@ -2365,7 +2367,8 @@ int rmb_sched_set_model(rmb_ctx* C, const float* params, uint32_t n_params, char
             if (!std::isfinite(params[i])) throw Fail(RMB_EINVAL, "schedule network parameters must be finite");
         CK(cudaSetDevice(C->p.device));
         C->sched_params.ensure(n_params * 4);
-        CK(cudaMemcpy(C->sched_params.p, params, n_params * 4, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(C->sched_params.p, params, n_params * 4, cudaMemcpyHostToDevice, C->st));
+        CK(cudaStreamSynchronize(C->st));
         C->sched_ready = true;
         return RMB_OK;
     } catch (const Fail& e) {
