@@ -1682,13 +1682,14 @@ __global__ void __launch_bounds__(256) k_prelim_prep(DevLib L, DevQueries Q, con
     }
 }
 
+// Blocks (subject, part of it).
 __global__ void __launch_bounds__(256) k_dp_subject(const uint8_t* __restrict__ plus, const uint64_t* __restrict__ off,
                                                     const uint32_t* __restrict__ len, uint8_t* __restrict__ out,
                                                     uint64_t stride) {
     const uint64_t o = off[blockIdx.x];
     const uint32_t n = len[blockIdx.x];
     uint8_t* d = out + o + (uint64_t)PACK_SPAD * (blockIdx.x + 1);
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.y * blockDim.x) {
         const uint8_t v = (uint8_t)((plus[o + 1 + i] & 15u) * 8u);
         d[i] = v;
         d[stride + n - 1 - i] = v;
@@ -2474,8 +2475,8 @@ __global__ void k_traceback_join(const DevParams* __restrict__ P, uint32_t n, co
     out[t] = o;
 }
 
-// Blocks a query in the kernels that go over every position of every query: one for 4,096 positions of a
-// query of the mean length.  (One block a query left a 2.1 Mb query to 512 threads: its lookup
+// Blocks a query (or a subject) in the kernels that go over every position of every one: one for 4,096 positions
+// of the mean length.  (One block a query left a 2.1 Mb query to 512 threads: its lookup
 // codes took 4.7 ms, 0.1 now, its reverse complement 4.6; a query of 60 kb 0.32 and 0.1.)
 static unsigned query_parts(uint64_t positions, uint32_t nq) {
     return (unsigned)std::min<uint64_t>(positions / nq / 4096 + 1, 1024);
@@ -2856,7 +2857,7 @@ cudaError_t launch_dp_subject(const uint8_t* plus, const uint64_t* off, const ui
     if (!n) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(out, 15 * 8, 2 * stride, st);
     if (e != cudaSuccess) return e;
-    k_dp_subject<<<n, 256, 0, st>>>(plus, off, len, out, stride);
+    k_dp_subject<<<dim3(n, query_parts(stride, n)), 256, 0, st>>>(plus, off, len, out, stride);
     return dp_pack(out, 2, stride, 3, nullptr, nullptr, st);
 }
 
